@@ -86,17 +86,25 @@ int eigh_jacobi(donof_ctx* ctx, cudaStream_t st, const double* G, int n, double*
 int iaux_f64(donof_ctx* ctx, cudaStream_t st, const double* G_host, const double* I_host, int nbf, int naux,
              double* b, DevBuf* part);
 
-// FP64-accurate T1 on the tensor cores from int8 digit slices (ozaki.cu):
-// ozaki_build makes the slices of the job's b (once), t1_ozaki computes
-// tmp[m + nbf*q + nbf*nbf5*l] = (B_l C5)[m, q]; transforms_f64 uses it whenever
-// the job holds the slices.
+// The FP64 form's contractions on the tensor cores from int8 digit slices
+// (ozaki.cu), used whenever the job holds b's slices (ozaki_build, once):
+// t1_ozaki computes tmp[m + nbf*q + nbf*nbf5*l] = (B_l C5)[m, q] in FP64;
+// transforms_ozaki leaves tmp as digit slices in job->tmp and b_pq in job->bpq;
+// y_ozaki then builds W's slices and leaves FP64 partials of Y in job->part (the
+// coefficients given to both must be the same).
 bool ozaki_shape_ok(int nbf);
 size_t ozaki_bytes(int nbf, int naux);
 int ozaki_build(donof_job* job);
 void ozaki_free(donof_job* job);
 int t1_ozaki(donof_job* job, cudaStream_t st, const double* C, int nbf5, double* tmp);
+int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
+                     const double* ck12, int nbf5);
+int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12, const double* ck12, int nbf5,
+            int nalpha, int nbeta, const double** ypart, int* nparts);
 
-// Tensor maps with 128-byte swizzle and zero fill (mixed.cu)
+// Tensor maps with zero fill (mixed.cu): 128-byte swizzle, or none (u64_flat)
+int make_tmap_u64_flat(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
+                       const cuuint64_t* strides_bytes, const cuuint32_t* box);
 int make_tmap_bf16(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
                    const cuuint64_t* strides_bytes, const cuuint32_t* box);
 int make_tmap_u8(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,

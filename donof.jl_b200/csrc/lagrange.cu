@@ -221,19 +221,18 @@ int grid_for(long long total, int threads, int sm) {
 
 }  // namespace
 
-// T1 + T2 into the job scratch: tmp (nbf x nbf5 x naux) and bpq (nbf5^2 x naux).
+// T1 + T2 into the job scratch: tmp (nbf x nbf5 x naux; digit slices of it with
+// b's digit slices on the device, see ozaki.cu) and bpq (nbf5^2 x naux).
 int transforms_f64(donof_job* job, cudaStream_t st, const double* C, int nbf5) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
+    if (job->oz_b) return transforms_ozaki(job, st, C, nullptr, nullptr, nullptr, nbf5);
     DONOF_CHECK(job->tmp.ensure(ctx, sizeof(double) * (size_t)nbf * nbf5 * naux));
     DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * nbf5 * naux));
     double* tmp = job->tmp.as<double>();
     double* bpq = job->bpq.as<double>();
     // T1: tmp_l(m,q) = sum_n b[m,n,l] C[n,q]; A(i=m,k=n) = b[m + nbf*n] (M-contiguous).
-    // With b's digit slices on the device it runs on the tensor cores (ozaki.cu).
-    if (job->oz_b) {
-        DONOF_CHECK(t1_ozaki(job, st, C, nbf5, tmp));
-    } else {
+    {
         GemmF64Args p{};
         p.M = nbf; p.N = nbf5; p.K = nbf;
         p.A = job->b; p.lda = nbf; p.strideA = (long long)nbf * nbf;
@@ -257,24 +256,37 @@ int transforms_f64(donof_job* job, cudaStream_t st, const double* C, int nbf5) {
     return DONOF_OK;
 }
 
-int lagrange2_f64(donof_job* job, cudaStream_t st, const double* C, const double* n,
-                  const double* H, const double* cj12, const double* ck12, int nbf5, int nalpha,
-                  int nbeta, double* elag, double* Hmat, double* E) {
+namespace {
+
+// Y = sum_{q,l} tmp[m, q + nbf5*l] W[q + nbf5*l, b], left as FP64 partials
+// (nbf x nbf5 each): the transforms, W and the split-K product, on the FP64 GEMM
+// or from digit slices on the tensor cores.
+int y_partials(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
+               const double* ck12, int nbf5, int nalpha, int nbeta, const double** ypart, int* nparts) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
+    if (job->oz_b) {
+        DONOF_CHECK(transforms_ozaki(job, st, C, n, cj12, ck12, nbf5));
+        return y_ozaki(job, st, n, cj12, ck12, nbf5, nalpha, nbeta, ypart, nparts);
+    }
     const long long Kt = (long long)nbf5 * naux;
-
     DONOF_CHECK(transforms_f64(job, st, C, nbf5));
-
     DONOF_CHECK(job->W.ensure(ctx, sizeof(double) * (size_t)Kt * (nbf5 + 1)));
     double* W = job->W.as<double>();
     DONOF_CHECK(build_w(ctx, st, job->bpq.as<double>(), n, cj12, ck12, nbf5, naux, nalpha, nbeta, W));
+    return gemm_f64_partials(ctx, st, false, true, nbf, nbf5, (int)Kt, job->tmp.as<double>(), nbf, W, Kt, &job->part,
+                             ypart, nparts);
+}
 
-    // Y = sum_{q,l} tmp[m, q + nbf5*l] W[q + nbf5*l, b], left as split-K partials
+}  // namespace
+
+int lagrange2_f64(donof_job* job, cudaStream_t st, const double* C, const double* n,
+                  const double* H, const double* cj12, const double* ck12, int nbf5, int nalpha,
+                  int nbeta, double* elag, double* Hmat, double* E) {
+    const int nbf = job->nbf;
     const double* ypart = nullptr;
     int nparts = 1;
-    DONOF_CHECK(gemm_f64_partials(ctx, st, false, true, nbf, nbf5, (int)Kt, job->tmp.as<double>(), nbf, W, Kt,
-                                  &job->part, &ypart, &nparts));
+    DONOF_CHECK(y_partials(job, st, C, n, cj12, ck12, nbf5, nalpha, nbeta, &ypart, &nparts));
     // H_mat = C^T (H C5) (src/utils.jl:17-18), elag = [n o H_mat + C^T Y | 0], E_elec
     return elag_tail_f64(job, st, C, H, n, nbf5, ypart, false, nparts, (long long)nbf * nbf5, Hmat, elag, E);
 }
@@ -287,16 +299,10 @@ int lagrange2_f64(donof_job* job, cudaStream_t st, const double* C, const double
 int lagrange2_partial_f64(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
                           const double* ck12, int nbf5, int nalpha, int nbeta, double* Y) {
     donof_ctx* ctx = job->ctx;
-    const int nbf = job->nbf, naux = job->naux;
-    const long long Kt = (long long)nbf5 * naux;
-    DONOF_CHECK(transforms_f64(job, st, C, nbf5));
-    DONOF_CHECK(job->W.ensure(ctx, sizeof(double) * (size_t)Kt * (nbf5 + 1)));
-    double* W = job->W.as<double>();
-    DONOF_CHECK(build_w(ctx, st, job->bpq.as<double>(), n, cj12, ck12, nbf5, naux, nalpha, nbeta, W));
+    const int nbf = job->nbf;
     const double* ypart = nullptr;
     int nparts = 1;
-    DONOF_CHECK(gemm_f64_partials(ctx, st, false, true, nbf, nbf5, (int)Kt, job->tmp.as<double>(), nbf, W, Kt,
-                                  &job->part, &ypart, &nparts));
+    DONOF_CHECK(y_partials(job, st, C, n, cj12, ck12, nbf5, nalpha, nbeta, &ypart, &nparts));
     const long long ny = (long long)nbf * nbf5;
     return splitk_reduce(ctx, st, ypart, ny, nparts, ny, Y, 0.0);
 }

@@ -644,11 +644,13 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 }  // namespace
 
-// Tensor map with 128-byte swizzle and zero fill outside the tensor (no
-// interleave): bf16 for the mixed kernels of this file and mixed_general.cu,
-// 8-bit for the digit slices of ozaki.cu.
+// Tensor map with zero fill outside the tensor (no interleave): bf16 with 128-byte
+// swizzle for the mixed kernels of this file and mixed_general.cu; for the digit
+// slices of ozaki.cu 8-bit with 128-byte swizzle, and 64-bit without swizzle
+// (16-byte core-matrix rows, two elements each).
 static int make_tmap(donof_ctx* ctx, CUtensorMap* map, CUtensorMapDataType dtype, const void* base, int rank,
-                     const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box);
+                     const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box,
+                     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
 int make_tmap_bf16(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
              const cuuint64_t* strides_bytes, const cuuint32_t* box) {
@@ -660,8 +662,15 @@ int make_tmap_u8(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, c
     return make_tmap(ctx, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, rank, dims, strides_bytes, box);
 }
 
+int make_tmap_u64_flat(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
+                       const cuuint64_t* strides_bytes, const cuuint32_t* box) {
+    return make_tmap(ctx, map, CU_TENSOR_MAP_DATA_TYPE_INT64, base, rank, dims, strides_bytes, box,
+                     CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 static int make_tmap(donof_ctx* ctx, CUtensorMap* map, CUtensorMapDataType dtype, const void* base, int rank,
-                     const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box) {
+                     const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box,
+                     CUtensorMapSwizzle swizzle) {
     auto fn = encode_fn();
     if (!fn) {
         set_error(ctx, "cuTensorMapEncodeTiled is not available");
@@ -669,7 +678,7 @@ static int make_tmap(donof_ctx* ctx, CUtensorMap* map, CUtensorMapDataType dtype
     }
     cuuint32_t es[5] = {1, 1, 1, 1, 1};
     CUresult r = fn(map, dtype, rank, const_cast<void*>(base), dims, strides_bytes, box, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error(ctx, "cuTensorMapEncodeTiled failed (%d)", (int)r);

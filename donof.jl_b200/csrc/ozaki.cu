@@ -1,34 +1,58 @@
-// FP64-accurate T1 (tmp_l = B_l C5, the first half of the b_mnP -> b_pqP
-// transform of src/utils.jl:19-20 and src/integrals.jl:150-152) on the
-// 5th-generation tensor cores, by exact integer products (the Ozaki scheme:
-// K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, "Error-free transformations of
-// matrix multiplication by using fast routines of matrix multiplication and
-// its applications", Numer. Algorithms 59 (2012) 95-118).
+// The FP64 form's three contractions on the 5th-generation tensor cores by
+// exact integer products (the Ozaki scheme: K. Ozaki, T. Ogita, S. Oishi,
+// S. M. Rump, "Error-free transformations of matrix multiplication by using
+// fast routines of matrix multiplication and its applications", Numer.
+// Algorithms 59 (2012) 95-118):
+//   T1   tmp_l  = B_l C5          (src/utils.jl:19-20, src/integrals.jl:150-152)
+//   T2   b_pq^l = C5^T tmp_l
+//   Y    Y      = sum_l tmp_l W_l  (the restructured Lagrangian of lagrange.cu)
 //
-// Every row m of B_l (over the contraction index n) and every column q of C5
-// is written as S = 7 signed 7-bit digits times a power of two,
-//     x = 2^e sum_{i<S} d_i 2^(-7(i+1)),   d_i in [-127, 127],
-// with 2^e the smallest power of two above the row's (column's) largest |x|:
-// d_i = trunc(128 r_i), r_(i+1) = 128 r_i - d_i, all exact in FP64, and the
-// residual is below 2^(-7S) 2^e.  Then
-//     tmp_l[m, q] = 2^(ea_m + eb_q) sum_g 2^(-7(g+2)) sum_{i+j=g} (D_i E_j)[m, q]
-// where each D_i E_j is an s8 x s8 GEMM whose int32 sums are exact
-// (tcgen05.mma kind::i8; |sum| <= 7 * 127^2 * nbf < 2^31 for nbf <= 16384).
-// The products with i + j >= S are dropped: they lie below the truncation
-// error.  That leaves 28 digit products in 7 int32 TMEM accumulators (one per
-// g, 64 columns each), combined in FP64 by the epilogue (exact int32 -> double,
-// Horner in 2^-7) and scaled by powers of two.  Since the C5 slices are adjacent in shared memory,
-// the products of one b slice with several C5 slices are one MMA of N = 64 x
-// (slices) <= 256: 10 MMAs per 32-wide step of n instead of 28.  The result differs from an FP64 GEMM by ~1e-13 of
-// the largest |tmp| (tests/test_gpu_ozaki.py states the bound).
+// Digits.  A number x with |x| <= F s (F = 0.498) is written as S signed 8-bit
+// digits, x = s sum_{i<S} d_i 256^-(i+1), d_i in [-128, 127]: with the integer
+// X = rint(x / s 2^(8S)) the bytes of X + sum_i 128 256^i are d_i + 128, so one
+// 64-bit addition yields every digit.  The residual is rounded to nearest
+// (no sign correlation between the dropped parts of the two operands), and the
+// scales are the largest |x| itself, not a power of two above it.
+//   b     6 digits, one scale per row m of b_l               (made once per job)
+//   C5    6 digits, one scale per column q                   (per call)
+//   tmp   7 digits, scale RL[l] CN[q]: the largest row norm of b_l times the norm
+//         of column q bounds |tmp_l[m, q]| (Cauchy-Schwarz), so the digits are
+//         written by T1's epilogue with no pass for a maximum; the bound is 2-3
+//         bits above the largest value, which the seventh digit pays for
+//   W     7 digits of RL[l] CN[q] W_l[q, b], one scale per b (beta_b times the
+//         largest |RL CN b_pq| and |RL CN t|, found by T2's epilogue and the
+//         diagonal kernel), so that tmp's scales drop out of Y's sum over (q, l)
+// A product keeps the digit pairs with i + j < G = 7: exact s8 x s8 -> s32 sums
+// (tcgen05.mma kind::i8) in 7 TMEM accumulators (one per i + j, 64 columns each),
+// combined in FP64 by the epilogue (exact int32 -> double, Horner in 2^-8).
+// |sum| <= 7 * 2^14 * K < 2^31 for K <= 18688; Y's K range is cut accordingly.
 //
-// b's digit slices are made once per job (it is constant); C5's per call.
-// One persistent kernel (ozaki_t1_kernel): a work unit is (aux index l,
-// 128-row tile of m); warp 8 streams b's slices (16 KB TMA boxes, no
-// multicast) through a ring, warp 9 issues the MMAs, warps 0-7 drain TMEM and
-// write tmp in FP64 in the layout the FP64 GEMM path writes.  Every wait is
-// bounded; on a timeout the CTA records the failure in the context's failure
-// word, drains its copies and MMAs, frees TMEM and exits.
+// One persistent kernel, oz_kernel<MODE>, with TMEM accumulators 7 x 64 columns
+// for a 128 x 64 output tile: warp 16 streams A's slices (16 KB TMA boxes, no
+// multicast) through a ring, warp 17 issues the MMAs, warps 0-15 drain TMEM.
+// B's slices are adjacent in shared memory, so the products of one A slice with
+// several B slices are one MMA of N = 64 x (slices) <= 256.
+//   T1: rows (m, l) flattened: no tile is cut at an aux index.  A = b's slices,
+//       B = C5's.
+//   T2: rows (q, l) flattened.  A = tmp's slices read MN-major, B = C5's.
+//   Y:  rows m, K = (q, l).  A = the same slices of tmp read K-major, B = W's;
+//       a unit is (tile, K range), its FP64 partial left for the tail to sum.
+// T1 and T2 keep the C5 slices of the CTA's column tile in shared memory for the
+// whole launch where they fit (nbf <= 384); a CTA then serves one column tile.
+//
+// Measured on one B200 (us; in brackets T1 from 7-bit digits, T2 and Y as FP64 GEMMs):
+//   nbf / naux / nbf5    T1            T2            W            Y            Lagrangian
+//   256 / 1024 / 64      104 (131)     40 (85)       21 (20)      32 (81)      (orbital step 289 (393))
+//   202 / 974 / 198      264 (470)     308 (761)     149 (186)    231 (841)    1029 (2231)
+//   384 / 1856 / 320     1700 (2049)   1541 (4649)   600 (698)    1266 (6958)  5848 (14295)
+// At nbf5 = 64 T1 is bound by HBM (b's slices in, tmp's out: 520 MB, 81 us at 6.45
+// TB/s); the larger ones by what the MMAs and the TMA need of shared memory (a
+// chunk of Y: 384 KB of operand reads, 168 KB written, 4300 cycles at 128 bytes a
+// cycle; 5100 measured) and, in T1 and T2, by the drain between two rounds.
+// The error against 64 bits fell from 7.2e-14 to 6.3e-15 of the norm of elag.
+//
+// Every wait is bounded; on a timeout the CTA records the failure in the
+// context's failure word, drains its copies and MMAs, frees TMEM and exits.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -43,47 +67,70 @@ namespace donof {
 
 namespace oz {
 
-constexpr int S = 7;                        // digit slices per operand
-constexpr int EPI_WARPS = 8;                // two per TMEM lane quarter, 32 columns each
-constexpr int PRODUCER = EPI_WARPS;         // warp 8: TMA producer
-constexpr int ISSUER = EPI_WARPS + 1;       // warp 9: TMEM allocator + MMA issuer
+constexpr int SB = 6;                       // digits of b and of C5
+constexpr int SW = 7;                       // digits of tmp and of W
+constexpr int NG = 7;                       // accumulators: digit pairs with i + j < NG
+constexpr double F = 0.498;                 // largest |x| / scale: every digit fits [-128, 127]
+constexpr int EPI_WARPS = 16;               // four per TMEM lane quarter, 16 columns each (8 of 32: T1 148 against 113 us at nbf5 = 64)
+constexpr int PRODUCER = EPI_WARPS;         // TMA producer
+constexpr int ISSUER = EPI_WARPS + 1;       // TMEM allocator + MMA issuer
 constexpr int NTHREADS = 32 * (EPI_WARPS + 2);
-constexpr int KC = 128;                     // n per stage: one 128-byte swizzle row of int8
-constexpr int MT = 128;                     // m rows per tile (MMA M)
-constexpr int QT = 64;                      // q columns per tile (MMA N per C5 slice)
-constexpr int A_BYTES = MT * KC;            // 16 KB: one slice of b over (m tile, n chunk)
-constexpr int BS_BYTES = QT * KC;           // 8 KB: one slice of C5 over (q tile, n chunk)
-constexpr int B_BYTES = S * BS_BYTES;       // 56 KB: every slice of C5 over (q tile, n chunk)
-constexpr int RING = 6;                     // b stages in flight (96 KB)
-constexpr int OFF_B = 0;                    // two C5 stages
-constexpr int OFF_RING = OFF_B + 2 * B_BYTES;
-constexpr int OFF_BAR = OFF_RING + RING * A_BYTES;
-constexpr int NBAR = 32;
-constexpr int OFF_MISC = OFF_BAR + NBAR * 8;  // tmem base, abort flag
-constexpr int SMEM_USED = OFF_MISC + 64;
-constexpr int SMEM_ALLOC = SMEM_USED + 1024;  // slack for 1024-B alignment
+// 18 warps put 5 on one SM sub-partition of 16384 registers: at most 96 per thread
+constexpr int BOUND_THREADS = 640;
+constexpr int KC = 128;                     // K per stage: one 128-byte swizzle row of int8
+constexpr int MT = 128;                     // rows per tile (MMA M)
+constexpr int QT = 64;                      // columns per tile (MMA N per B slice)
+constexpr int A_BYTES = MT * KC;            // 16 KB: one slice of A over (row tile, K chunk)
+constexpr int BS_BYTES = QT * KC;           // 8 KB: one slice of B over (column tile, K chunk)
+constexpr int RING_MAX = 8;                 // A stages in flight
+constexpr int OFF_BAR = 0;
+constexpr int OFF_MISC = 512;               // tmem base, abort flag
+constexpr int OFF_DATA = 1024;              // B stages, then the A ring
+constexpr int DATA_BYTES = 224 * 1024;
+constexpr int SMEM_ALLOC = OFF_DATA + DATA_BYTES + 1024;  // slack for 1024-B alignment
 static_assert(SMEM_ALLOC <= 227 * 1024, "shared memory budget");
-static_assert(S * QT <= 512, "TMEM columns");
+static_assert(NG * QT <= 512, "TMEM columns");
+constexpr int KMAX_CHUNKS = 146;            // 7 * 2^14 * 146 * 128 < 2^31
+static_assert(7ll * 16384 * KMAX_CHUNKS * KC < (1ll << 31), "int32 accumulators");
 
 // barrier indices
-constexpr int A_FULL = 0;               // +s (RING): b stage landed
-constexpr int A_EMPTY = RING;           // +s: b stage consumed by the MMAs
-constexpr int B_FULL = 2 * RING;        // +slot (2): C5 stage landed
-constexpr int B_EMPTY = B_FULL + 2;     // +slot: C5 stage consumed
-constexpr int ACC_FULL = B_EMPTY + 2;   // every accumulator of a round (unit, q tile) complete
-constexpr int GFREE = ACC_FULL + 1;     // +g (S): accumulator g drained and zeroed (count EPI_WARPS)
-constexpr int B_END = GFREE + S;        // every MMA of the CTA complete
-static_assert(B_END < NBAR, "barrier count");
+constexpr int A_FULL = 0;                   // +s (RING_MAX): A stage landed
+constexpr int A_EMPTY = RING_MAX;           // +s: A stage consumed by the MMAs
+constexpr int B_FULL = 2 * RING_MAX;        // +stage: B stage landed (resident: one per K chunk)
+constexpr int B_STAGES = 8;
+constexpr int B_EMPTY = B_FULL + B_STAGES;  // +slot (2): streamed B stage consumed
+constexpr int ACC_FULL = B_EMPTY + 2;       // accumulators of a round complete: +0 the last (6), +1 5..3, +2 2..0
+constexpr int GFREE = ACC_FULL + 3;         // +g (NG): accumulator g drained and zeroed (count EPI_WARPS)
+constexpr int B_END = GFREE + NG;           // every MMA of the CTA complete
+static_assert((B_END + 1) * 8 <= OFF_MISC, "barrier area");
+
+enum Mode {
+    T1_DIGITS = 0,  // tmp as digit slices
+    T1_F64 = 1,     // tmp in FP64
+    T2 = 2,         // b_pq in FP64
+    YSUM = 3,       // FP64 partials of Y
+};
 
 struct Params {
-    int nbf, nbf5, naux;
-    int nmt, nkc, nqt;   // tiles of m (128), chunks of n (128), tiles of q (64)
-    int resident;        // nqt * nkc <= 2: every C5 stage is loaded once and kept
-    const double* sa;    // 2^ea per (m, l): sa[m + nbf*l]
-    const double* sb;    // 2^(eb - 14) per q
-    double* tmp;         // tmp[m + nbf*q + nbf*nbf5*l]
-    int* fail;           // the context's failure word for mbarrier waits
-    long long wait;      // cycle budget of every bounded wait (drains excepted)
+    int nbf, nbf5, naux, ldq;  // ldq: nbf5 rounded up to 16 (row length of tmp's and W's slices per l)
+    int nrt, nct;              // row tiles (128), column tiles (64)
+    int nkc;                   // K chunks (128): all of T1's and T2's range, the whole (q, l) range for Y
+    int cpu, nsplit;           // Y: chunks per unit, units per tile
+    int k4_last;               // 32-wide K steps of the last chunk
+    int resident;              // B's stages of the CTA's column tile are loaded once and kept
+    int ring;                  // A stages
+    int ring_off;              // byte offset of the ring behind OFF_DATA
+    const double* ra;          // sa / RL per row (m, l) of b
+    const double* RL;          // per l
+    const double* CN;          // per q
+    const double* cb;          // per q: sb 2^40 / CN
+    const double* sb2;         // per q: sb 2^-16
+    const double* beta;        // per b (Y)
+    unsigned* wmax;            // [0] of |RL CN b_pq|, [1] of |RL CN t| / beta: high words of the largest value
+    int8_t* t8;                // tmp's slices (see the layout above t8_at)
+    double* out;               // FP64 output
+    int* fail;                 // the context's failure word for mbarrier waits
+    long long wait;            // cycle budget of every bounded wait (drains excepted)
 };
 
 using namespace sm100;
@@ -95,34 +142,221 @@ __device__ __forceinline__ double exact_f64(int x) {
     return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0;
 }
 
-// Round r of a CTA = one (unit, q tile): its MMAs accumulate into the 7
-// accumulators, then the epilogue drains them.  The b slices of an n chunk are
-// consumed from the least significant (i = 6) to the most (i = 0): slice i
-// writes accumulators i .. 6 only, so the first MMAs of round r + 1 need only
-// accumulator 6, which the epilogue of round r drains (and zeroes) first.  The
-// drain of accumulator g is a TMEM load and a store of zeros; its release
-// (GFREE[g]) comes right after, and the FP64 arithmetic of the epilogue runs
-// while the next round's MMAs already fill the released columns.
-__global__ void __launch_bounds__(NTHREADS, 1)
-ozaki_t1_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                const Params P) {
+// Layout of the slices (the MMAs read them without swizzle): 128-wide chunks of the
+// contiguous index (R = q + ldq l of tmp and W, n of b and C5), each in eight groups
+// of 16, a group's 16 bytes contiguous and the rows one 16-byte step apart.
+//   b    b8[n % 16 + 16 (r % 128 + 128 (n / 16 + ldn/16 (i + 6 (r / 128))))]   r = m + nbf l
+//   tmp  t8[R % 16 + 16 (m + nbf (g + 8 (i + 7 chunk)))]      g = R / 16 % 8, chunk = R / 128
+//   W    w8[R % 16 + 16 (b + nbf5 (j + 7 (g + 8 chunk)))]
+//   C5   c8[n % 16 + 16 (q + nbf5 (j + 6 (g + 8 chunk)))]
+// A row step of 16 bytes makes the stores contiguous over a warp's rows (512 bytes an
+// instruction: with rows 128 bytes apart W's kernel took 185 instead of 126 us at
+// nbf5 = 198), gives the 8 x 16-byte core matrices that a K-major and an MN-major
+// operand share, and W's and C5's digits lie one after the other along N for every
+// group.  A box is rows of 2 KB: T1's loads alone took 234 us at nbf = 202 as 128
+// swizzled rows of 128 bytes at a pitch of 208, and take 160 us so.
+__device__ __forceinline__ size_t t8_at(int R, int m, int nbf) {  // digit 0; digit i: + 128 nbf i
+    return 16 * ((size_t)nbf * ((size_t)(R >> 7) * 8 * SW + ((R >> 4) & 7)) + m) + (R & 15);
+}
+
+// The seven digits of z (|z| <= F 2^56) as bytes: byte 6 - i is digit i.
+__device__ __forceinline__ unsigned long long digits7(double z) {
+    const unsigned long long bias = 0x0080808080808080ull;
+    return (unsigned long long)(__double2ll_rn(z) + (long long)bias) ^ bias;
+}
+
+// Byte transposition of four 7-byte digit strings: w[i] = digit i of z0, z1, z2, z3.
+__device__ __forceinline__ void pack4(const unsigned long long (&z)[4], unsigned (&w)[SW]) {
+    const unsigned a0 = (unsigned)z[0], a1 = (unsigned)z[1], a2 = (unsigned)z[2], a3 = (unsigned)z[3];
+    const unsigned h0 = (unsigned)(z[0] >> 32), h1 = (unsigned)(z[1] >> 32), h2 = (unsigned)(z[2] >> 32),
+                   h3 = (unsigned)(z[3] >> 32);
+    unsigned t0 = __byte_perm(a0, a1, 0x5140), t1 = __byte_perm(a2, a3, 0x5140);
+    w[6] = __byte_perm(t0, t1, 0x5410);
+    w[5] = __byte_perm(t0, t1, 0x7632);
+    t0 = __byte_perm(a0, a1, 0x7362);
+    t1 = __byte_perm(a2, a3, 0x7362);
+    w[4] = __byte_perm(t0, t1, 0x5410);
+    w[3] = __byte_perm(t0, t1, 0x7632);
+    t0 = __byte_perm(h0, h1, 0x5140);
+    t1 = __byte_perm(h2, h3, 0x5140);
+    w[2] = __byte_perm(t0, t1, 0x5410);
+    w[1] = __byte_perm(t0, t1, 0x7632);
+    t0 = __byte_perm(h0, h1, 0x7362);
+    t1 = __byte_perm(h2, h3, 0x7362);
+    w[0] = __byte_perm(t0, t1, 0x5410);
+}
+
+// 32 bytes in one store (dst 32-byte aligned)
+__device__ __forceinline__ void store_f64x4(double* dst, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// |x| <= value_above(high word of |x|): the bits of the next high word (NaN for a
+// NaN or an infinity).
+__device__ __forceinline__ double value_above(unsigned hi) {
+    return __hiloint2double((int)(hi < 0x7ff00000u ? hi + 1u : 0x7ff80000u), 0);
+}
+
+// The scale of W's digits over F: beta_b M with M an upper bound of the
+// largest |RL CN W| / beta (NaN when a term was not finite); 0 when W's row is zero.
+__device__ __forceinline__ double w_scale(double beta, const unsigned* wmax) {
+    double M = (value_above(wmax[0]) + value_above(wmax[1])) * (1.0 + 0x1p-40);
+    if (M < 1e-280) M = 1e-280;
+    double s = beta * M;
+    if (s < 1e-290) s = 0.0;
+    return s;
+}
+
+// The work of one CTA: unit u = (row tile, column tile, K range).
+struct Unit {
+    int row, col;  // tile indices
+    int c0, nc;    // K chunks [c0, c0 + nc)
+    int split;
+};
+
+template <int MODE, bool RES>
+__device__ __forceinline__ int unit_count(const Params& P) {
+    const int c = blockIdx.x, G = gridDim.x;
+    if (MODE == YSUM) {
+        const int n = P.nrt * P.nct * P.nsplit;
+        return (n - c + G - 1) / G;
+    }
+    if (RES) {  // CTA c serves column tile c % nct, every (G of that tile)-th row tile
+        const int ct = c % P.nct, gc = (G - ct + P.nct - 1) / P.nct, r0 = c / P.nct;
+        return r0 < P.nrt ? (P.nrt - r0 + gc - 1) / gc : 0;
+    }
+    const int n = P.nrt * P.nct;
+    return (n - c + G - 1) / G;
+}
+
+template <int MODE, bool RES>
+__device__ __forceinline__ Unit unit_of(const Params& P, int u) {
+    const int c = blockIdx.x, G = gridDim.x;
+    Unit w;
+    w.c0 = 0;
+    w.nc = P.nkc;
+    w.split = 0;
+    if (MODE == YSUM) {
+        const int i = c + u * G, tiles = P.nrt * P.nct;
+        w.split = i / tiles;
+        const int t = i - w.split * tiles;
+        w.row = t % P.nrt;
+        w.col = t / P.nrt;
+        w.c0 = w.split * P.cpu;
+        w.nc = min(P.cpu, P.nkc - w.c0);
+    } else if (RES) {
+        const int ct = c % P.nct, gc = (G - ct + P.nct - 1) / P.nct;
+        w.row = c / P.nct + u * gc;
+        w.col = ct;
+    } else {
+        const int i = c + u * G;
+        w.row = i / P.nct;
+        w.col = i - w.row * P.nct;
+    }
+    return w;
+}
+
+// One elected lane's MMAs of A slice i (stage at descriptor ad) with B slices 0 ..
+// cnt-1 (stage at bd) over nk4 steps of 32 K: accumulators i .. i + cnt - 1, as one
+// MMA of N = 64 cnt or two (7 = 4 + 3, 6 = 3 + 3, 5 = 3 + 2); part 1 the lower of the
+// two, part 2 the upper, 3 both.  `done` (0: none) is the barrier that the commit
+// behind them arrives on.  i and part are constants after unrolling; the branch on
+// nk4 stays outside the elected lane's region, which is straight code (an MMA takes
+// about 80 issue cycles, 92 to execute: what the warp does between them counts).
+template <int MODE, int NB>
+__device__ __forceinline__ void issue_slice(int i, int part, uint32_t tmem, uint64_t ad, uint64_t bd, int nk4,
+                                            uint32_t done) {
+    const int cnt = (NG - i) < NB ? (NG - i) : NB;
+    const int first = cnt <= 4 ? cnt : (cnt + 1) / 2;
+    // 32 K further: two groups, or for the MN-major operand four 8-row core matrices
+    constexpr uint64_t astep = (MODE == T2 ? 32 * 16 : 2 * 16 * MT) >> 4;
+    constexpr uint64_t bstep = (2 * 16 * NB * QT) >> 4;
+    constexpr uint32_t amn = MODE == T2 ? 1u << 15 : 0u;
+    auto step = [&](int k4) {
+        if (part & 1)
+            umma_i8(tmem + (uint32_t)(i * QT), ad + k4 * astep, bd + k4 * bstep, idesc_i8(MT, QT * first) | amn, 1u);
+        if ((part & 2) && cnt > first)
+            umma_i8(tmem + (uint32_t)((i + first) * QT), ad + k4 * astep, bd + k4 * bstep + (uint64_t)(first * QT),
+                    idesc_i8(MT, QT * (cnt - first)) | amn, 1u);
+    };
+    if (nk4 == 4) {
+        if (elect_one()) {
+            step(0); step(1); step(2); step(3);
+            if (done) umma_commit(done);
+        }
+    } else if (nk4 == 3) {
+        if (elect_one()) {
+            step(0); step(1); step(2);
+            if (done) umma_commit(done);
+        }
+    } else if (nk4 == 2) {
+        if (elect_one()) {
+            step(0); step(1);
+            if (done) umma_commit(done);
+        }
+    } else {
+        if (elect_one()) {
+            step(0);
+            if (done) umma_commit(done);
+        }
+    }
+    __syncwarp();
+}
+
+// Descriptors of an A stage and of a B stage.
+template <int MODE>
+__device__ __forceinline__ uint64_t a_desc(uint32_t addr) {
+    if (MODE == T2) return sdesc_flat(addr, 128, 16 * MT);  // MN-major: (q, l) along M, 8 m per 128 bytes
+    return sdesc_flat(addr, 16 * MT, 128);                  // K-major: groups of 16 K 2 KB apart
+}
+template <int NB>
+__device__ __forceinline__ uint64_t b_desc(uint32_t addr) {
+    return sdesc_flat(addr, 16 * NB * QT, 128);
+}
+
+// Round r of a CTA = one unit: its MMAs accumulate into the 7 accumulators, then
+// the epilogue drains them.  A's slices are consumed from the least significant
+// (i = NA - 1) to the most: slice i writes accumulators i .. 6 only, so the first
+// MMAs of round r + 1 need only the top accumulators, which the epilogue of round
+// r drains (and zeroes) first.  The drain of accumulator g is a TMEM load and a
+// store of zeros; its release (GFREE[g]) comes right after, and the FP64
+// arithmetic of the epilogue runs while the next round's MMAs already fill the
+// released columns.
+// With B resident (NKC = its K chunks, 1 to 3) the order is slice-major over the K
+// chunks, and a round ends with slice 0 against B's upper slices (accumulators 5..3),
+// then its lower ones (2..0): accumulator 6 is complete a slice earlier, 5..3 half a
+// slice earlier, so the epilogue drains them while the last MMAs run and the tensor
+// cores do not wait for it between rounds.  With B streamed (NKC = 0) the order is
+// chunk by chunk.
+template <int MODE, int NKC>
+__global__ void __launch_bounds__(BOUND_THREADS, 1)
+oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params P) {
+    constexpr int NA = (MODE == T2 || MODE == YSUM) ? SW : SB;
+    constexpr int NB = (MODE == YSUM) ? SW : SB;
+    constexpr int B_BYTES = NB * BS_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t sbase = saddr(sm);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
+    const uint32_t sbase = saddr(sm) + OFF_DATA;
+    const uint32_t sring = sbase + (uint32_t)P.ring_off;
+    const uint32_t sbar = saddr(sm) + OFF_BAR;
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_MISC);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_MISC + 16);
-    auto bar = [&](int i) { return saddr(&bars[i]); };
+    auto bar = [&](int i) { return sbar + 8u * (uint32_t)i; };
+    auto wait_on = [&](uint32_t b, uint32_t parity) {  // of a whole warp
+        bool r = mbar_try(b, parity);
+        if (!__all_sync(0xffffffffu, r)) r = mbar_wait(b, parity, abort_flag, P.wait);
+        return __all_sync(0xffffffffu, r) != 0;
+    };
+    auto wait = [&](int i, uint32_t parity) { return wait_on(bar(i), parity); };
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int G = gridDim.x;
-    const int nunits = P.naux * P.nmt;
-    const int my_units = (nunits - (int)blockIdx.x + G - 1) / G;  // unit w = blockIdx.x + u*G
-    const int nbst = P.nqt * P.nkc;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    constexpr bool resident = NKC > 0;
+    const int my_units = unit_count<MODE, resident>(P);
+    static_assert(!(resident && NB == NG), "accumulator 6 must be complete before slice 0");
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        for (int i = 0; i <= B_END; ++i) mbar_init(bar(i), (i >= GFREE && i < GFREE + S) ? EPI_WARPS : 1);
+        for (int i = 0; i <= B_END; ++i) mbar_init(bar(i), (i >= GFREE && i < GFREE + NG) ? EPI_WARPS : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == ISSUER) {
@@ -136,235 +370,298 @@ ozaki_t1_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
     if (warp == PRODUCER) {
         // ------------------------------------------------------------ producer
-        // b's slices in the order the MMAs consume them: with C5 resident, slice
-        // i of every n chunk before slice i-1 (i = S-1 .. 0), so that a round
-        // needs accumulator 0 only for its last nkc stages; with C5 streamed, per
-        // q tile and n chunk the C5 stage, then the slices i = S-1 .. 0
-        if (lane == 0 && my_units > 0) {
-            int it = 0, bs = 0;
+        // Every lane of the warp waits, one elected lane issues (a wait by lane 0
+        // alone, broadcast to the others, took 560 cycles a stage instead of 75).
+        if (my_units > 0) {
+            int it = 0, s = 0, bs = 0;  // A stages issued, their slot, B stages issued
+            uint32_t ph = 1;            // parity of the slot's "consumed" phase
             bool ok = true;
-            if (P.resident) {
-                for (int b = 0; b < nbst; ++b) {
-                    const int qt = b / P.nkc, kc = b - qt * P.nkc;
-                    mbar_expect_tx(bar(B_FULL + b), (uint32_t)B_BYTES);
-                    tma_load_3d(sbase + OFF_B + b * B_BYTES, &map_b, bar(B_FULL + b), kc * KC, qt * QT, 0);
+            auto load_a = [&](int i, int kc, int row) {
+                if (!wait(A_EMPTY + s, ph)) return false;
+                if (elect_one()) {
+                    mbar_expect_tx(bar(A_FULL + s), (uint32_t)A_BYTES);
+                    if (MODE == T2)  // 128 m (K) of the 128 (q, l) of a row tile
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * kc * KC, 0, i + SW * row);
+                    else if (MODE == YSUM)  // 128 (q, l) (K) of 128 m
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * row * MT, 0, i + SW * kc);
+                    else  // 128 n (K) of 128 (m, l)
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 0, 8 * kc, i + SB * row);
                 }
+                __syncwarp();
+                ++it;
+                if (++s == P.ring) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+                return true;
+            };
+            auto load_b = [&](int stage, int col, int kc) {
+                if (elect_one()) {
+                    mbar_expect_tx(bar(B_FULL + stage), (uint32_t)B_BYTES);
+                    tma_load_3d(sbase + stage * B_BYTES, &map_b, bar(B_FULL + stage), 2 * col * QT, 0, 8 * kc);
+                }
+                __syncwarp();
+            };
+            if (resident) {
+                const int col = unit_of<MODE, resident>(P, 0).col;
+                for (int kc = 0; kc < P.nkc; ++kc) load_b(kc, col, kc);
             }
             for (int u = 0; u < my_units && ok; ++u) {
-                const int w = (int)blockIdx.x + u * G;
-                const int l = w / P.nmt, mt = w - l * P.nmt;
-                for (int qt = 0; qt < P.nqt && ok; ++qt) {
-                    if (P.resident) {
-                        for (int i = S - 1; i >= 0 && ok; --i)
-                            for (int kc = 0; kc < P.nkc; ++kc, ++it) {
-                                const int s = it % RING;
-                                if (!mbar_wait(bar(A_EMPTY + s), (uint32_t)(((it / RING) & 1) ^ 1), abort_flag, P.wait)) {
-                                    ok = false;
-                                    break;
-                                }
-                                mbar_expect_tx(bar(A_FULL + s), (uint32_t)A_BYTES);
-                                tma_load_4d(sbase + OFF_RING + s * A_BYTES, &map_a, bar(A_FULL + s), kc * KC, mt * MT, i, l);
-                            }
-                        continue;
+                const Unit w = unit_of<MODE, resident>(P, u);
+                if (resident) {
+                    for (int i = NA - 1; i >= 0 && ok; --i)
+                        for (int kc = 0; kc < w.nc && ok; ++kc) ok = load_a(i, kc, w.row);
+                    continue;
+                }
+                for (int kc = w.c0; kc < w.c0 + w.nc && ok; ++kc, ++bs) {
+                    const int slot = bs & 1;
+                    if (!wait(B_EMPTY + slot, (uint32_t)(((bs >> 1) & 1) ^ 1))) {
+                        ok = false;
+                        break;
                     }
-                    for (int kc = 0; kc < P.nkc && ok; ++kc) {
-                        if (!P.resident) {
-                            const int slot = bs & 1;
-                            if (!mbar_wait(bar(B_EMPTY + slot), (uint32_t)(((bs >> 1) & 1) ^ 1), abort_flag, P.wait)) {
-                                ok = false;
-                                break;
-                            }
-                            mbar_expect_tx(bar(B_FULL + slot), (uint32_t)B_BYTES);
-                            tma_load_3d(sbase + OFF_B + slot * B_BYTES, &map_b, bar(B_FULL + slot), kc * KC, qt * QT, 0);
-                            ++bs;
-                        }
-                        for (int i = S - 1; i >= 0; --i, ++it) {
-                            const int s = it % RING;
-                            if (!mbar_wait(bar(A_EMPTY + s), (uint32_t)(((it / RING) & 1) ^ 1), abort_flag, P.wait)) {
-                                ok = false;
-                                break;
-                            }
-                            mbar_expect_tx(bar(A_FULL + s), (uint32_t)A_BYTES);
-                            tma_load_4d(sbase + OFF_RING + s * A_BYTES, &map_a, bar(A_FULL + s), kc * KC, mt * MT, i, l);
-                        }
-                    }
+                    load_b(slot, w.col, kc);
+                    for (int i = NA - 1; i >= 0 && ok; --i) ok = load_a(i, kc, w.row);
                 }
             }
             // drain: every issued copy has landed before the CTA exits
-            for (int j = (it > RING ? it - RING : 0); j < it; ++j)
-                mbar_drain(bar(A_FULL + j % RING), (uint32_t)((j / RING) & 1));
-            if (P.resident) {
-                for (int b = 0; b < nbst; ++b) mbar_drain(bar(B_FULL + b), 0);
+            for (int j = (it > P.ring ? it - P.ring : 0); j < it; ++j)
+                mbar_drain(bar(A_FULL + j % P.ring), (uint32_t)((j / P.ring) & 1));
+            if (resident) {
+                for (int kc = 0; kc < P.nkc; ++kc) mbar_drain(bar(B_FULL + kc), 0);
             } else {
-                for (int j = (bs > 2 ? bs - 2 : 0); j < bs; ++j) mbar_drain(bar(B_FULL + (j & 1)), (uint32_t)((j >> 1) & 1));
+                for (int j = (bs > 2 ? bs - 2 : 0); j < bs; ++j)
+                    mbar_drain(bar(B_FULL + (j & 1)), (uint32_t)((j >> 1) & 1));
             }
         }
     } else if (warp == ISSUER) {
         // ------------------------------------------------------------ MMA issuer
         // accumulator g (TMEM columns [64 g, 64 g + 64)) collects D_i E_j, i + j = g.
-        // The C5 slices lie one after the other in shared memory (slice j = rows
+        // The B slices lie one after the other in shared memory (slice j = rows
         // [64 j, 64 j + 64) of the stage), so D_i times slices j0 .. j0+c-1 is ONE
         // MMA with N = 64 c whose columns land on accumulators i+j0 .. i+j0+c-1.
         // The epilogue zeroes every accumulator it releases: all MMAs accumulate.
-        if (lane == 0 && my_units > 0) {
-            int s = 0, bs = 0, rnd = 0;  // ring slot of the next b stage, C5 stages, rounds
-            uint32_t aph = 0;            // phase of the ring's current pass
+        // The whole warp runs the loop, one elected lane issues.
+        if (my_units > 0) {
+            // ring position: the full barrier and descriptor of the next stage, what is
+            // left of the pass, its phase; the empty barriers lie RING_MAX behind
+            uint32_t fb = bar(A_FULL), aph = 0;
+            uint64_t ad = a_desc<MODE>(sring);
+            int left = P.ring, bs = 0;
             bool ok = true;
+            bool ready = false;  // this lane saw the next A stage land
+            bool gready = false; // ... and the next accumulator released
+            auto next = [&]() {  // to the next stage, whose arrival is asked for while MMAs are issued
+                fb += 8u;
+                ad += A_BYTES >> 4;
+                if (--left == 0) {
+                    fb = bar(A_FULL);
+                    ad = a_desc<MODE>(sring);
+                    left = P.ring;
+                    aph ^= 1u;
+                }
+                ready = mbar_test(fb, aph);
+            };
+            auto landed = [&]() {
+                if (!__all_sync(0xffffffffu, ready) && !wait_on(fb, aph)) return false;
+                return true;
+            };
             for (int u = 0; u < my_units && ok; ++u) {
-                for (int qt = 0; qt < P.nqt && ok; ++qt, ++rnd) {
-                    if (P.resident) {
-                        const uint64_t bq = sdesc(sbase + OFF_B + qt * P.nkc * B_BYTES, 16, 1024);
-                        if (rnd == 0)
-                            for (int b = 0; b < nbst && ok; ++b) ok = mbar_wait(bar(B_FULL + b), 0, abort_flag, P.wait);
-                        fence_after();
+                const uint32_t up = (uint32_t)(u & 1);
+                if constexpr (resident) {
+                    if (u == 0)
 #pragma unroll
-                        for (int ii = 0; ii < S; ++ii) {
-                            const int i = S - 1 - ii;
-                            for (int kc = 0; kc < P.nkc && ok; ++kc) {
-                                const uint64_t bd = bq + (uint64_t)((kc * B_BYTES) >> 4);
-                                if (kc == 0 && !mbar_wait(bar(GFREE + i), (uint32_t)(rnd & 1), abort_flag, P.wait)) {
-                                    ok = false;
-                                    break;
-                                }
-                                if (!mbar_wait(bar(A_FULL + s), aph, abort_flag, P.wait)) {
-                                    ok = false;
-                                    break;
-                                }
-                                fence_after();
-                                const uint64_t ad = sdesc(sbase + OFF_RING + s * A_BYTES, 16, 1024);
+                        for (int kc = 0; kc < NKC; ++kc) ok = ok && wait(B_FULL + kc, 0);
 #pragma unroll
-                                for (int k4 = 0; k4 < KC / 32; ++k4) {
+                    for (int ii = 0; ii < NA; ++ii) {
+                        const int i = NA - 1 - ii;
+                        if (ii == 0)
+                            for (int g = NG - 1; g >= i; --g) ok = ok && wait(GFREE + g, up);
+                        else if (!__all_sync(0xffffffffu, gready))
+                            ok = ok && wait(GFREE + i, up);
+                        uint32_t db[NKC];
+                        uint64_t da[NKC];
 #pragma unroll
-                                    for (int j0 = 0; j0 < S - i; j0 += 4) {
-                                        constexpr int kMax = 4;
-                                        const int cnt = (S - i - j0) < kMax ? (S - i - j0) : kMax;
-                                        umma_i8(tmem + (uint32_t)((i + j0) * QT), ad + (uint64_t)(2 * k4),
-                                                bd + (uint64_t)((j0 * BS_BYTES + k4 * 32) >> 4), idesc_i8(MT, QT * cnt), 1u);
-                                    }
-                                }
-                                umma_commit(bar(A_EMPTY + s));
-                                if (++s == RING) {
-                                    s = 0;
-                                    aph ^= 1u;
-                                }
-                            }
+                        for (int kc = 0; kc < NKC; ++kc) {
+                            ok = ok && landed();
                             if (!ok) break;
-                        }
-                        if (!ok) break;
-                        umma_commit(bar(ACC_FULL));
-                        continue;
-                    }
-                    for (int kc = 0; kc < P.nkc && ok; ++kc) {
-                        const int bslot = P.resident ? qt * P.nkc + kc : (bs & 1);
-                        const uint32_t bpar = P.resident ? 0u : (uint32_t)((bs >> 1) & 1);
-                        if (!mbar_wait(bar(B_FULL + bslot), bpar, abort_flag, P.wait)) {
-                            ok = false;
-                            break;
-                        }
-                        fence_after();
-                        // descriptors are linear in the shared-memory address (addr >> 4 in the
-                        // low 14 bits, no carry below 256 KB): offsets are plain adds
-                        const uint64_t bd = sdesc(sbase + OFF_B + bslot * B_BYTES, 16, 1024);
-#pragma unroll
-                        for (int ii = 0; ii < S; ++ii) {
-                            const int i = S - 1 - ii;
-                            // accumulator i (and, released before it, i+1 .. 6) free for this round
-                            if (kc == 0 && !mbar_wait(bar(GFREE + i), (uint32_t)(rnd & 1), abort_flag, P.wait)) {
-                                ok = false;
-                                break;
-                            }
-                            if (!mbar_wait(bar(A_FULL + s), aph, abort_flag, P.wait)) {
-                                ok = false;
-                                break;
-                            }
+                            const uint32_t done = fb + 8u * RING_MAX;
+                            const uint64_t d = ad;
+                            next();
+                            if (i > 0 && kc == NKC - 1) gready = mbar_test(bar(GFREE + i - 1), up);
                             fence_after();
-                            const uint64_t ad = sdesc(sbase + OFF_RING + s * A_BYTES, 16, 1024);
-#pragma unroll
-                            for (int k4 = 0; k4 < KC / 32; ++k4) {
-#pragma unroll
-                                for (int j0 = 0; j0 < S - i; j0 += 4) {
-                                    constexpr int kMax = 4;  // N = 64 cnt <= 256
-                                    const int cnt = (S - i - j0) < kMax ? (S - i - j0) : kMax;
-                                    umma_i8(tmem + (uint32_t)((i + j0) * QT), ad + (uint64_t)(2 * k4),
-                                            bd + (uint64_t)((j0 * BS_BYTES + k4 * 32) >> 4), idesc_i8(MT, QT * cnt), 1u);
-                                }
-                            }
-                            umma_commit(bar(A_EMPTY + s));
-                            if (++s == RING) {
-                                s = 0;
-                                aph ^= 1u;
+                            const uint64_t bd = b_desc<NB>(sbase + kc * B_BYTES);
+                            const int nk4 = kc == NKC - 1 ? P.k4_last : KC / 32;
+                            if (i > 0) {
+                                issue_slice<MODE, NB>(i, 3, tmem, d, bd, nk4, done);
+                            } else {
+                                issue_slice<MODE, NB>(0, 2, tmem, d, bd, nk4, 0);
+                                db[kc] = done;
+                                da[kc] = d;
                             }
                         }
                         if (!ok) break;
-                        if (!P.resident) {
-                            umma_commit(bar(B_EMPTY + bslot));
-                            ++bs;
+                        if (i == 1) {
+                            if (elect_one()) umma_commit(bar(ACC_FULL));
+                            __syncwarp();
+                        } else if (i == 0) {
+                            if (elect_one()) umma_commit(bar(ACC_FULL + 1));
+                            __syncwarp();
+#pragma unroll
+                            for (int kc = 0; kc < NKC; ++kc)
+                                issue_slice<MODE, NB>(0, 1, tmem, da[kc], b_desc<NB>(sbase + kc * B_BYTES),
+                                                      kc == NKC - 1 ? P.k4_last : KC / 32, db[kc]);
+                            if (elect_one()) umma_commit(bar(ACC_FULL + 2));
+                            __syncwarp();
                         }
                     }
-                    if (!ok) break;
-                    umma_commit(bar(ACC_FULL));
+                } else {
+                    const Unit w = unit_of<MODE, resident>(P, u);
+                    for (int g = NG - 1; g >= 0; --g) ok = ok && wait(GFREE + g, up);
+                    for (int kc = w.c0; kc < w.c0 + w.nc && ok; ++kc, ++bs) {
+                        const int slot = bs & 1;
+                        const uint64_t bd = b_desc<NB>(sbase + slot * B_BYTES);
+                        const int nk4 = kc == P.nkc - 1 ? P.k4_last : KC / 32;
+                        ok = wait(B_FULL + slot, (uint32_t)((bs >> 1) & 1));
+#pragma unroll
+                        for (int ii = 0; ii < NA; ++ii) {
+                            ok = ok && landed();
+                            if (!ok) break;
+                            const uint32_t done = fb + 8u * RING_MAX;
+                            const uint64_t d = ad;
+                            next();
+                            fence_after();
+                            issue_slice<MODE, NB>(NA - 1 - ii, 3, tmem, d, bd, nk4, done);
+                        }
+                        if (ok && elect_one()) umma_commit(bar(B_EMPTY + slot));
+                        __syncwarp();
+                    }
+                    if (ok && elect_one()) {
+                        umma_commit(bar(ACC_FULL));
+                        umma_commit(bar(ACC_FULL + 1));
+                        umma_commit(bar(ACC_FULL + 2));
+                    }
+                    __syncwarp();
                 }
             }
-            umma_commit(bar(B_END));
+            if (elect_one()) umma_commit(bar(B_END));
+            __syncwarp();
             mbar_drain(bar(B_END), 0);  // every MMA of this CTA has completed
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 0-7)
-        // warp w reads TMEM lanes [32 (w % 4), +32) = rows m = 128 mt + 32 (w % 4) + lane,
-        // and columns [32 (w / 4), +32) of every accumulator = q = 64 qt + 32 (w / 4) + k
-        const int quarter = warp & 3, half = warp >> 2;
-        const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 32);
-        // zero every accumulator and release it for the first work unit
+        // ------------------------------------------------------------ epilogue (warps 0-15)
+        // warp w reads TMEM lanes [32 (w % 4), +32) = rows 128 row + 32 (w % 4) + lane,
+        // and columns [16 (w / 4), +16) of every accumulator
+        constexpr int NC = QT / 4;
+        const int quarter = warp & 3, group = warp >> 2;
+        const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * NC);
+        // zero every accumulator and release it for the first round
 #pragma unroll
-        for (int g = 0; g < S; ++g) tmem_zero32(tl + (uint32_t)(g * QT));
+        for (int g = 0; g < NG; ++g) tmem_zero16(tl + (uint32_t)(g * QT));
         tmem_wait_st();
         fence_before();
         __syncwarp();
         if (lane == 0)
-            for (int g = 0; g < S; ++g) mbar_arrive(bar(GFREE + g));
-        int rnd = 0;
-        bool ok = true;
-        for (int u = 0; u < my_units && ok; ++u) {
-            const int w = (int)blockIdx.x + u * G;
-            const int l = w / P.nmt, mt = w - l * P.nmt;
-            const int m = mt * MT + quarter * 32 + lane;
-            const bool mrow = m < P.nbf;
-            const double sa = mrow ? P.sa[m + (size_t)P.nbf * l] : 0.0;
-            double* dst = P.tmp + (size_t)P.nbf * P.nbf5 * l + m;
-            for (int qt = 0; qt < P.nqt; ++qt, ++rnd) {
-                int r = 1;
-                if (lane == 0) r = mbar_wait(bar(ACC_FULL), (uint32_t)(rnd & 1), abort_flag, P.wait) ? 1 : 0;
-                r = __shfl_sync(0xffffffffu, r, 0);
-                if (!r) {
-                    ok = false;
-                    break;
+            for (int g = 0; g < NG; ++g) mbar_arrive(bar(GFREE + g));
+        unsigned top = 0;  // T2: largest high word of |RL CN b_pq| of this thread
+        for (int u = 0; u < my_units; ++u) {
+            const Unit w = unit_of<MODE, resident>(P, u);
+            const int R = w.row * MT + quarter * 32 + lane;
+            const int q0 = w.col * QT + group * NC;
+            // per-row data, read before the wait
+            int l = 0, x = 0;  // aux index, and m (T1) or q (T2)
+            bool in;
+            double rs = 0.0;
+            if (MODE == YSUM) {
+                x = R;
+                in = R < P.nbf;
+            } else if (MODE == T2) {
+                l = R / P.ldq;
+                x = R - l * P.ldq;
+                in = l < P.naux && x < P.nbf5;
+                if (in) rs = P.RL[l] * P.CN[x];
+            } else {
+                l = R / P.nbf;
+                x = R - l * P.nbf;
+                in = l < P.naux;
+                if (in) rs = MODE == T1_F64 ? P.ra[R] * P.RL[l] : P.ra[R];
+            }
+            // Horner in 2^-8 from the least significant accumulator: v = sum_g acc_g 2^(-8g)
+            double v[NC];
+            bool ok = true;
+#pragma unroll
+            for (int g = NG - 1; g >= 0; --g) {
+                if (g == 6 || g == 5 || g == 2) {
+                    ok = ok && wait(ACC_FULL + (g == 6 ? 0 : g == 5 ? 1 : 2), (uint32_t)(u & 1));
+                    if (!ok) break;
+                    fence_after();
                 }
-                fence_after();
-                // Horner in 2^-7 from the least significant accumulator: v = sum_g acc_g 2^(-7g)
-                double v[32];
+                uint32_t a[NC];
+                tmem_issue16(tl + (uint32_t)(g * QT), a);
+                tmem_wait_ld();
+                tmem_zero16(tl + (uint32_t)(g * QT));
+                tmem_wait_st();
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(GFREE + g));
 #pragma unroll
-                for (int g = S - 1; g >= 0; --g) {
-                    uint32_t a[32];
-                    tmem_issue32(tl + (uint32_t)(g * QT), a);
-                    tmem_wait_ld();
-                    tmem_zero32(tl + (uint32_t)(g * QT));
-                    tmem_wait_st();
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(GFREE + g));
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const double x = exact_f64((int)a[k]);
-                        v[k] = (g == S - 1) ? x : fma(v[k], 0x1p-7, x);
-                    }
-                }
-                const int q0 = qt * QT + half * 32;
-#pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const int q = q0 + k;
-                    if (mrow && q < P.nbf5) dst[(size_t)P.nbf * q] = v[k] * sa * P.sb[q];
+                for (int k = 0; k < NC; ++k) {
+                    const double t = exact_f64((int)a[k]);
+                    v[k] = (g == NG - 1) ? t : fma(v[k], 0x1p-8, t);
                 }
             }
+            if (!ok) break;
+            if (MODE == T1_DIGITS) {
+                // digit slices of tmp, q contiguous: 16 bytes per slice and thread; the
+                // padding columns [nbf5, ldq) get cb = 0, i.e. zero digits
+                unsigned wd[4][SW];
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) {
+                    unsigned long long z[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) z[k] = digits7(v[4 * k4 + k] * (rs * P.cb[q0 + 4 * k4 + k]));
+                    pack4(z, wd[k4]);
+                }
+                if (in && q0 < P.ldq) {
+                    int8_t* dst = P.t8 + t8_at(P.ldq * l + q0, x, P.nbf);
+#pragma unroll
+                    for (int i = 0; i < SW; ++i)
+                        *reinterpret_cast<uint4*>(dst + (size_t)i * P.nbf * 128) =
+                            make_uint4(wd[0][i], wd[1][i], wd[2][i], wd[3][i]);
+                }
+            } else if (MODE == T1_F64) {
+                double* dst = P.out + (size_t)P.nbf * P.nbf5 * l + x;
+#pragma unroll
+                for (int k = 0; k < NC; ++k)
+                    if (in && q0 + k < P.nbf5) dst[(size_t)P.nbf * (q0 + k)] = v[k] * rs * P.sb2[q0 + k];
+            } else if (MODE == T2) {
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    v[k] = v[k] * rs * P.sb2[q0 + k];  // b_pq (columns at and beyond nbf5: sb2 = 0)
+                    if (in) top = max(top, (unsigned)__double2hiint(v[k] * rs) & 0x7fffffffu);
+                }
+                double* dst = P.out + ((size_t)P.nbf5 * l + x) * P.nbf5 + q0;
+                if (in && q0 + NC <= P.nbf5 && (P.nbf5 & 3) == 0) {
+#pragma unroll
+                    for (int k = 0; k < NC; k += 4) store_f64x4(dst + k, v[k], v[k + 1], v[k + 2], v[k + 3]);
+                } else if (in && q0 + NC <= P.nbf5 && (P.nbf5 & 1) == 0) {
+#pragma unroll
+                    for (int k = 0; k < NC; k += 2) *reinterpret_cast<double2*>(dst + k) = make_double2(v[k], v[k + 1]);
+                } else if (in) {
+#pragma unroll
+                    for (int k = 0; k < NC; ++k)
+                        if (q0 + k < P.nbf5) dst[k] = v[k];
+                }
+            } else {
+                double* dst = P.out + (size_t)w.split * P.nbf * P.nbf5 + x;
+#pragma unroll
+                for (int k = 0; k < NC; ++k)
+                    if (in && q0 + k < P.nbf5)
+                        dst[(size_t)P.nbf * (q0 + k)] = v[k] * (w_scale(P.beta[q0 + k], P.wmax) * (0x1p-16 / F));
+            }
+        }
+        if (MODE == T2) {
+            for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+            if (lane == 0) atomicMax(P.wmax, top);
         }
     }
 
@@ -378,36 +675,63 @@ ozaki_t1_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 }
 
 // ---------------------------------------------------------------- digit slices
-// Row scales of b: sa[m + nbf*l] = 2^e with max_n |b[m, n, l]| < 2^e (1 for a
-// zero row); one thread per (m, l), coalesced over m.
-__global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long long naux, double* __restrict__ sa) {
+// The six digits of x / s (|x| <= F s) as bytes: byte 5 - i is digit i.
+__device__ __forceinline__ unsigned long long digits6(double x, double s) {
+    const unsigned long long bias = 0x0000808080808080ull;
+    return (unsigned long long)(__double2ll_rn(x / s * 0x1p48) + (long long)bias) ^ bias;
+}
+
+// The digit scale of a row or column whose largest |x| is mx (floored, so that
+// x / s never overflows; a zero row has zero digits whatever its scale).
+__device__ __forceinline__ double digit_scale(double mx) { return fmax(mx, 1e-280) / F; }
+
+// Per row (m, l) of b: sa = digit_scale(max_n |b|) into ra (made sa / RL by
+// row_finish_kernel) and the row norm's maximum over m into rn[l] (bits of a
+// non-negative double).  One thread per (m, l), coalesced over m.
+__global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long long naux, double* __restrict__ ra,
+                                 unsigned long long* __restrict__ rn) {
     const long long total = (long long)nbf * naux;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         const long long l = i / nbf;
         const int m = (int)(i - l * nbf);
         const double* row = b + (long long)nbf * nbf * l + m;
-        double mx = 0.0;
-        for (int n = 0; n < nbf; ++n) mx = fmax(mx, fabs(row[(long long)nbf * n]));
-        int e = 0;
-        if (mx > 0.0) frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1)
-        sa[i] = ldexp(1.0, e);
+        double mx = 0.0, ss = 0.0;
+        for (int n = 0; n < nbf; ++n) {
+            const double x = fabs(row[(long long)nbf * n]);
+            mx = fmax(mx, x);
+            ss += x * x;
+        }
+        double norm = sqrt(ss);
+        if (mx > 0.0 && !(ss > 1e-250 && ss < 1e250)) {  // squares out of range: scaled by the maximum
+            ss = 0.0;
+            for (int n = 0; n < nbf; ++n) {
+                const double x = row[(long long)nbf * n] / mx;
+                ss += x * x;
+            }
+            norm = mx * sqrt(ss);
+        }
+        ra[i] = digit_scale(mx);
+        atomicMax(rn + l, (unsigned long long)__double_as_longlong(norm));
     }
 }
 
-// Digits of one value scaled into (-1, 1): d_i = trunc(128 r_i), r_(i+1) = 128 r_i - d_i.
-__device__ __forceinline__ void digits(double y, int8_t (&d)[S]) {
-#pragma unroll
-    for (int i = 0; i < S; ++i) {
-        y *= 128.0;
-        const double t = trunc(y);
-        d[i] = (int8_t)(int)t;
-        y -= t;
+// rn[l] (bits) -> RL[l] = norm (1 + 2^-30) / F in place, ra = sa / RL (0 for b_l = 0)
+__global__ void row_finish_kernel(int nbf, long long naux, const unsigned long long* __restrict__ rn,
+                                  double* __restrict__ RL, double* __restrict__ ra) {
+    const long long total = (long long)nbf * naux;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long l = i / nbf;
+        const double R = __longlong_as_double((long long)rn[l]) * (1.0 + 0x1p-30) / F;
+        if (i == l * nbf) RL[l] = R;
+        ra[i] = R > 0.0 ? ra[i] / R : 0.0;
     }
 }
 
-// b's slices, transposed so that n is contiguous: out[n + ldn*(m + nbf*(i + S*l))].
-// 32 x 32 (m, n) tiles through shared memory: reads coalesced over m, writes over n.
+// b's slices (layout above t8_at), n < ldn = nbf rounded up to 16.  32 x 32 (m, n)
+// tiles through shared memory: reads coalesced over m, four n of one digit a 4-byte
+// word.  s = digit_scale of the row.
 __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__ b, const double* __restrict__ sa,
                                                       int nbf, int ldn, long long naux, int8_t* __restrict__ out) {
     __shared__ double tile[32][33];
@@ -426,46 +750,204 @@ __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__
             tile[ty + 8 * k][tx] = (m < nbf && n < nbf) ? B[m + (long long)nbf * n] : 0.0;  // tile[n][m]
         }
         __syncthreads();
+        // a warp: 8 m of 4 words (16 n)
+        const int m = m0 + (ty & 3) * 8 + (tx >> 2), nq = 16 * (ty >> 2) + 4 * (tx & 3);
+        if (m < nbf && n0 + nq < ldn) {  // ldn is a multiple of 16: whole words
+            const double s = sa[m + (long long)nbf * l];
+            unsigned long long z[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int m = m0 + ty + 8 * k, n = n0 + tx;
-            if (m >= nbf || n >= nbf) continue;
-            int8_t d[S];
-            digits(tile[tx][ty + 8 * k] / sa[m + (long long)nbf * l], d);
+            for (int k = 0; k < 4; ++k) z[k] = digits6(tile[nq + k][m - m0], s) << 8;
+            unsigned w[SW];
+            pack4(z, w);  // digit i of the 6 is byte 6 - i of the shifted string
+            const long long row = m + (long long)nbf * l;
+            int8_t* dst = out + 16 * ((row & 127) + 128 * (((n0 + nq) >> 4) + (long long)(ldn / 16) * SB * (row >> 7))) + (nq & 15);
 #pragma unroll
-            for (int i = 0; i < S; ++i) out[n + (long long)ldn * (m + (long long)nbf * (i + S * l))] = d[i];
+            for (int i = 0; i < SB; ++i) *reinterpret_cast<unsigned*>(dst + 128ll * ldn * i) = w[i];
         }
     }
 }
 
-// C5's slices (one block per column q): sb[q] = 2^(e - 14) with max_n |C[n, q]| < 2^e,
-// out[n + ldn*(q + nbf5*i)].
-__global__ void __launch_bounds__(256) split_c_kernel(const double* __restrict__ C, int nbf, int nbf5, int ldn,
-                                                      double* __restrict__ sb, int8_t* __restrict__ out) {
-    __shared__ double red[8];
-    __shared__ double inv_s;
-    const int q = blockIdx.x;
-    const double* col = C + (long long)nbf * q;
-    double mx = 0.0;
-    for (int n = threadIdx.x; n < nbf; n += blockDim.x) mx = fmax(mx, fabs(col[n]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
-        int e = 0;
-        if (m > 0.0) frexp(m, &e);
-        sb[q] = ldexp(1.0, e - 14);  // 2^-14: the weight 2^(-7(i+1) - 7(j+1)) of digit pair (0, 0)
-        inv_s = ldexp(1.0, -e);
+struct PrepArgs {
+    const double* C;
+    const double *n, *cj12, *ck12;  // null: no W will be built
+    int nbf, nbf5, nkc;             // grid: the columns rounded up to whole tiles
+    double *sb2, *CN, *cb, *beta;
+    int8_t* out;                    // c8, n padded to whole chunks with zeros
+    unsigned* wmax;
+};
+
+// One block per column q of C5 (and per padding column): its digit slices, the
+// scales of T1 and T2, and beta_q = the largest |factor| of W's column q.
+__global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
+    __shared__ double red[3][4];
+    __shared__ double bc[3];
+    const int q = blockIdx.x, tid = threadIdx.x;
+    if (q == 0 && tid < 2) a.wmax[tid] = 0;
+    if (q >= a.nbf5) {
+        if (tid == 0) a.sb2[q] = a.CN[q] = a.cb[q] = a.beta[q] = 0.0;
+        return;
     }
-    __syncthreads();
-    const double inv = inv_s;
-    for (int n = threadIdx.x; n < nbf; n += blockDim.x) {
-        int8_t d[S];
-        digits(col[n] * inv, d);
+    const double* col = a.C + (long long)a.nbf * q;
+    double mx = 0.0, be = 0.0;
+    for (int n = tid; n < a.nbf; n += blockDim.x) mx = fmax(mx, fabs(col[n]));
+    bool bad = false;
+    if (a.n != nullptr) {
+        for (int p = tid; p < a.nbf5; p += blockDim.x) {
+            const double x = a.cj12[q + (long long)a.nbf5 * p], y = a.ck12[q + (long long)a.nbf5 * p];
+            be = fmax(be, fmax(fabs(x), fabs(y)));
+            bad = bad || isnan(x) || isnan(y);
+        }
+        const double x = a.n[q];
+        be = fmax(be, fabs(x));
+        bad = bad || isnan(x);
+    }
+    auto reduce = [&](double x, int k, bool sum) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_xor_sync(0xffffffffu, x, o);
+            x = sum ? x + y : fmax(x, y);
+        }
+        if ((tid & 31) == 0) red[k][tid >> 5] = x;
+        __syncthreads();
+        if (tid == 0) {
+            double t = red[k][0];
+            for (int w = 1; w < 4; ++w) t = sum ? t + red[k][w] : fmax(t, red[k][w]);
+            bc[k] = t;
+        }
+        __syncthreads();
+        return bc[k];
+    };
+    mx = reduce(mx, 0, false);
+    be = reduce(be, 1, false);
+    const bool anybad = __syncthreads_or(bad);
+    const double s = digit_scale(mx);
+    double ss = 0.0;
+    for (int n = tid; n < a.nbf; n += blockDim.x) {
+        const double x = col[n] / s;
+        ss += x * x;
+    }
+    ss = reduce(ss, 2, true);
+    if (tid == 0) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        double cn = s * sqrt(ss) * (1.0 + 0x1p-40);
+        if (!isfinite(ss) || isinf(mx)) cn = nan;  // a column with a NaN or an infinity: every product of it is NaN
+        a.CN[q] = cn;
+        a.sb2[q] = isnan(cn) ? nan : s * 0x1p-16;
+        a.cb[q] = cn == 0.0 ? 0.0 : s * 0x1p40 / cn;
+        a.beta[q] = anybad ? nan : be;
+    }
+    for (int n = tid; n < a.nkc * KC; n += blockDim.x) {
+        const unsigned long long z = n < a.nbf ? digits6(col[n], s) : 0ull;
+        int8_t* dst = a.out + (n & 15) + 16 * (q + (long long)a.nbf5 * SB * (n >> 4));
 #pragma unroll
-        for (int i = 0; i < S; ++i) out[n + (long long)ldn * (q + (long long)nbf5 * i)] = d[i];
+        for (int i = 0; i < SB; ++i) dst[16ll * a.nbf5 * i] = (int8_t)(z >> (8 * (SB - 1 - i)));
+    }
+}
+
+// ---------------------------------------------------------------- W
+// tv[b + nbf5 l] = n'_b d_b^l + sum_q cj12[b, q] d_q^l with d_q^l = b_pq^l[q, q]
+// (lagrange.cu), and the largest |RL CN tv| / beta.  A block takes 32 b of LB aux
+// indices: the diagonals staged in shared memory a panel of DQ at a time, each of
+// its eight warps on an eighth of the panel's q (one cj12 element, read along b,
+// serves LB products), the eight partial sums added in a fixed order.
+constexpr int LB = 8;
+constexpr int DQ = 256;
+
+__global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ bpq, const double* __restrict__ n,
+                                                   const double* __restrict__ cj12, int nbf5, int naux, int nalpha,
+                                                   int nbeta, const double* __restrict__ RL,
+                                                   const double* __restrict__ CN, const double* __restrict__ beta,
+                                                   double* __restrict__ tv, unsigned* __restrict__ wmax) {
+    __shared__ double sd[DQ * LB];       // [q][LB]
+    __shared__ double part[8][LB][32];   // [warp][l][b]
+    const int l0 = blockIdx.x * LB, b = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
+    const long long n55 = (long long)nbf5 * nbf5;
+    double s[LB];
+#pragma unroll
+    for (int k = 0; k < LB; ++k) s[k] = 0.0;
+    for (int p0 = 0; p0 < nbf5; p0 += DQ) {
+        const int np = min(DQ, nbf5 - p0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < LB * np; i += blockDim.x) {
+            const int k = i / np, q = i - k * np;
+            sd[q * LB + k] = l0 + k < naux ? bpq[n55 * (l0 + k) + (long long)(p0 + q) * (nbf5 + 1)] : 0.0;
+        }
+        __syncthreads();
+        if (b < nbf5) {
+#pragma unroll 4
+            for (int q = warp; q < np; q += 8) {
+                const double c = cj12[b + (long long)nbf5 * (p0 + q)];
+#pragma unroll
+                for (int k = 0; k < LB; ++k) s[k] = fma(c, sd[q * LB + k], s[k]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < LB; ++k) part[warp][k][threadIdx.x & 31] = s[k];
+    __syncthreads();
+    unsigned top = 0;
+    const int l = l0 + warp;  // warp k finishes aux index l0 + k (LB warps)
+    if (b < nbf5 && l < naux) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][warp][threadIdx.x & 31];
+        const bool dj = (nbeta > 0) && (b < nbeta || b >= nalpha);
+        if (dj) t = fma(n[b], bpq[n55 * l + (long long)b * (nbf5 + 1)], t);
+        tv[b + (long long)nbf5 * l] = t;
+        const double be = beta[b];
+        top = (unsigned)__double2hiint(RL[l] * t * (be == 0.0 ? 0.0 : CN[b] / be)) & 0x7fffffffu;
+    }
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(wmax + 1, top);
+}
+static_assert(LB == 8, "one warp per aux index of a block");
+
+// W's digit slices (layout at t8_at, R = q + ldq l) of RL CN W_l[q, b] over its scale,
+// W_l[q, b] = -ck12[b, q] b_pq^l[b, q] + delta_qb tv.
+// A thread takes 16 q of one (b, l): 16 loads in flight, coalesced over b, and one
+// 16-byte store per slice, contiguous over b; zero digits in the padding
+// (q >= nbf5, and R beyond the last aux index: tmp's slices are not written there).
+__global__ void __launch_bounds__(256) w_digits_kernel(const double* __restrict__ bpq, const double* __restrict__ ck12,
+                                                       const double* __restrict__ tv, int nbf5, int naux, int ldq,
+                                                       int nch, const double* __restrict__ RL,
+                                                       const double* __restrict__ CN, const double* __restrict__ beta,
+                                                       const unsigned* __restrict__ wmax, int8_t* __restrict__ W8) {
+    const int nbp = (nbf5 + 31) / 32 * 32;
+    const long long total = (long long)nbp * nch * 8, n55 = (long long)nbf5 * nbf5;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int t = (int)(i / nbp);  // 16 values of R
+        const int b = (int)(i - (long long)t * nbp);
+        const int l = 16 * t / ldq, q0 = 16 * t - l * ldq;
+        if (b >= nbf5) continue;
+        const bool in = l < naux;
+        const double* B = bpq + n55 * l + b;
+        double v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = in && q0 + k < nbf5 ? B[(long long)nbf5 * (q0 + k)] : 0.0;
+        const double sc = w_scale(beta[b], wmax);
+        const double f = (sc == 0.0 || !in) ? 0.0 : RL[l] * (F * 0x1p56 / sc);
+        const double td = (in && b >= q0 && b < q0 + 16) ? tv[b + (long long)nbf5 * l] : 0.0;
+        unsigned wd[4][SW];
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+            unsigned long long z[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = q0 + 4 * k4 + k;
+                double x = 0.0;
+                if (q < nbf5) {
+                    x = -ck12[b + (long long)nbf5 * q] * v[4 * k4 + k];
+                    if (q == b) x += td;
+                    x *= CN[q];
+                }
+                z[k] = digits7(x * f);
+            }
+            pack4(z, wd[k4]);
+        }
+        int8_t* dst = W8 + 16 * ((long long)nbf5 * SW * t + b);
+#pragma unroll
+        for (int j = 0; j < SW; ++j)
+            *reinterpret_cast<uint4*>(dst + 16ll * nbf5 * j) = make_uint4(wd[0][j], wd[1][j], wd[2][j], wd[3][j]);
     }
 }
 
@@ -474,16 +956,182 @@ __global__ void __launch_bounds__(256) split_c_kernel(const double* __restrict__
 namespace {
 
 int ldn_of(int nbf) { return (nbf + 15) / 16 * 16; }  // 16-byte row pitch (TMA stride rule)
-size_t slice_bytes(int nbf, int naux) { return (size_t)naux * oz::S * nbf * ldn_of(nbf); }
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+// one slice of b (whole 128-row tiles); the job's buffer holds the SB slices, one
+// slice's worth of workspace (W's digit slices, where they fit), ra and RL
+size_t slice_bytes(int nbf, int naux) { return ((size_t)naux * nbf + oz::MT - 1) / oz::MT * oz::MT * ldn_of(nbf); }
+
+struct JobLayout {
+    size_t work, ra, rl, bytes;
+};
+JobLayout job_layout(int nbf, int naux) {
+    JobLayout o;
+    o.work = align256(oz::SB * slice_bytes(nbf, naux));
+    o.ra = o.work + align256(slice_bytes(nbf, naux));
+    o.rl = o.ra + align256(sizeof(double) * (size_t)nbf * naux);
+    o.bytes = o.rl + sizeof(double) * 2 * (size_t)naux;  // RL, and the bits of the row norms
+    return o;
+}
+
+// C5's slices and the per-column arrays of a call, in job->oz_c
+struct CallLayout {
+    int nq;
+    size_t sb2, cn, cb, beta, wmax, bytes;
+};
+CallLayout call_layout(int nbf, int nbf5) {
+    CallLayout o;
+    o.nq = (nbf5 + oz::QT - 1) / oz::QT * oz::QT;
+    const size_t col = align256(sizeof(double) * (size_t)o.nq);
+    o.sb2 = align256((size_t)oz::SB * nbf5 * ((nbf + oz::KC - 1) / oz::KC * oz::KC));
+    o.cn = o.sb2 + col;
+    o.cb = o.cn + col;
+    o.beta = o.cb + col;
+    o.wmax = o.beta + col;
+    o.bytes = o.wmax + 256;
+    return o;
+}
+
+int ldq_of(int nbf5) { return (nbf5 + 15) / 16 * 16; }
+// 128-wide chunks of the (q, l) index
+int chunks_of(int nbf5, int naux) { return (int)(((long long)ldq_of(nbf5) * naux + oz::KC - 1) / oz::KC); }
+
+template <int MODE, int NKC>
+int launch_one(donof_ctx* ctx, cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, const oz::Params& P,
+               int grid) {
+    static std::atomic<unsigned long long> attr_mask{0};
+    const unsigned long long bit = 1ull << (ctx->device & 63);
+    if (!(attr_mask.load(std::memory_order_acquire) & bit)) {
+        DONOF_CUDA(ctx, cudaFuncSetAttribute(oz::oz_kernel<MODE, NKC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             oz::SMEM_ALLOC));
+        attr_mask.fetch_or(bit, std::memory_order_acq_rel);
+    }
+    oz::oz_kernel<MODE, NKC><<<grid, oz::NTHREADS, oz::SMEM_ALLOC, st>>>(ma, mb, P); count_launch();
+    DONOF_CUDA(ctx, cudaGetLastError());
+    return DONOF_OK;
+}
+// The instance for the call's resident K chunks (0: B streamed).
+template <int MODE>
+int launch_oz(donof_ctx* ctx, cudaStream_t st, const CUtensorMap& ma, const CUtensorMap& mb, const oz::Params& P,
+              int grid) {
+    if constexpr (MODE != oz::YSUM) {
+        if (P.resident && P.nkc == 1) return launch_one<MODE, 1>(ctx, st, ma, mb, P, grid);
+        if (P.resident && P.nkc == 2) return launch_one<MODE, 2>(ctx, st, ma, mb, P, grid);
+        if (P.resident && P.nkc == 3) return launch_one<MODE, 3>(ctx, st, ma, mb, P, grid);
+    }
+    return launch_one<MODE, 0>(ctx, st, ma, mb, P, grid);
+}
+
+// Parameters common to the products of a call.
+oz::Params base_params(donof_job* job, int nbf5) {
+    donof_ctx* ctx = job->ctx;
+    const JobLayout jl = job_layout(job->nbf, job->naux);
+    const CallLayout cl = call_layout(job->nbf, nbf5);
+    char* jb = static_cast<char*>(job->oz_b);
+    char* cb = job->oz_c.as<char>();
+    oz::Params P{};
+    P.nbf = job->nbf; P.nbf5 = nbf5; P.naux = job->naux; P.ldq = ldq_of(nbf5);
+    P.ra = reinterpret_cast<double*>(jb + jl.ra);
+    P.RL = reinterpret_cast<double*>(jb + jl.rl);
+    P.sb2 = reinterpret_cast<double*>(cb + cl.sb2);
+    P.CN = reinterpret_cast<double*>(cb + cl.cn);
+    P.cb = reinterpret_cast<double*>(cb + cl.cb);
+    P.beta = reinterpret_cast<double*>(cb + cl.beta);
+    P.wmax = reinterpret_cast<unsigned*>(cb + cl.wmax);
+    P.fail = ctx->fail_dev ? ctx->fail_dev + FAIL_MBAR : nullptr;
+    P.wait = sm100::wait_budget(ctx->wait_limit);
+    return P;
+}
+
+// Tiles, ring and CTAs of a product with K = nbf and C5's slices as B (T1, T2):
+// B stays in shared memory where its column tile and at least four A stages fit
+// (nbf <= 384) and every column tile has a CTA, else it streams through two stages.
+int shape_c5(donof_ctx* ctx, oz::Params& P, long long rows) {
+    constexpr int stage = oz::SB * oz::BS_BYTES;
+    P.nrt = (int)((rows + oz::MT - 1) / oz::MT);
+    P.nct = (P.nbf5 + oz::QT - 1) / oz::QT;
+    P.nkc = (P.nbf + oz::KC - 1) / oz::KC;
+    P.k4_last = (P.nbf - (P.nkc - 1) * oz::KC + 31) / 32;
+    const long long units = (long long)P.nrt * P.nct;
+    const int grid = (int)(units < ctx_ctas(ctx) ? units : ctx_ctas(ctx));
+    P.resident = P.nkc <= 3 && P.nkc * stage + 4 * oz::A_BYTES <= oz::DATA_BYTES && grid >= P.nct;
+    P.ring_off = (P.resident ? P.nkc : 2) * stage;
+    P.ring = (oz::DATA_BYTES - P.ring_off) / oz::A_BYTES;
+    if (P.ring > oz::RING_MAX) P.ring = oz::RING_MAX;
+    return grid;
+}
+
+// rows x digits of 16-byte groups (C5's slices, W's slices): boxes of 64 rows, every
+// digit, the eight groups of a chunk
+int map_b(donof_job* job, const void* base, int rows, int digits, int chunks, CUtensorMap* m) {
+    cuuint64_t dims[3] = {2 * (cuuint64_t)rows, (cuuint64_t)digits, 8 * (cuuint64_t)chunks};
+    cuuint64_t strides[2] = {16 * (cuuint64_t)rows, 16 * (cuuint64_t)rows * digits};
+    cuuint32_t box[3] = {2 * oz::QT, (cuuint32_t)digits, 8};
+    return make_tmap_u64_flat(job->ctx, m, base, 3, dims, strides, box);
+}
+int map_c5(donof_job* job, int nbf5, CUtensorMap* m) {
+    return map_b(job, job->oz_c.ptr, nbf5, oz::SB, (job->nbf + oz::KC - 1) / oz::KC, m);
+}
+
+// tmp's slices: T2's A operand (MN-major) and Y's (K-major) share the map: boxes of
+// 128 m, the eight groups of a chunk of (q, l), one digit
+int map_t8(donof_job* job, int nbf5, CUtensorMap* m) {
+    const cuuint64_t nbf = job->nbf;
+    cuuint64_t dims[3] = {2 * nbf, 8, (cuuint64_t)oz::SW * chunks_of(nbf5, job->naux)};
+    cuuint64_t strides[2] = {16 * nbf, 128 * nbf};
+    cuuint32_t box[3] = {2 * oz::MT, 8, 1};
+    return make_tmap_u64_flat(job->ctx, m, job->tmp.ptr, 3, dims, strides, box);
+}
+
+// C5's slices and scales (and W's beta where the coefficients are given)
+int prep(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12, const double* ck12,
+         int nbf5) {
+    donof_ctx* ctx = job->ctx;
+    const CallLayout cl = call_layout(job->nbf, nbf5);
+    DONOF_CHECK(job->oz_c.ensure(ctx, cl.bytes));
+    const oz::Params P = base_params(job, nbf5);
+    oz::PrepArgs a{};
+    a.C = C; a.n = n; a.cj12 = cj12; a.ck12 = ck12;
+    a.nbf = job->nbf; a.nbf5 = nbf5; a.nkc = (job->nbf + oz::KC - 1) / oz::KC;
+    a.sb2 = const_cast<double*>(P.sb2); a.CN = const_cast<double*>(P.CN); a.cb = const_cast<double*>(P.cb);
+    a.beta = const_cast<double*>(P.beta);
+    a.out = job->oz_c.as<int8_t>(); a.wmax = P.wmax;
+    oz::prep_kernel<<<cl.nq, 128, 0, st>>>(a); count_launch();
+    DONOF_CUDA(ctx, cudaGetLastError());
+    return DONOF_OK;
+}
+
+// T1 of the call's C5: tmp's digit slices into job->tmp, or tmp in FP64 into `out`.
+int t1(donof_job* job, cudaStream_t st, int nbf5, double* out) {
+    donof_ctx* ctx = job->ctx;
+    const int nbf = job->nbf, naux = job->naux, ldn = ldn_of(nbf);
+    CUtensorMap ma, mb;
+    {   // b's slices: boxes of 128 rows (m, l), the eight groups of a chunk of n, one digit
+        const cuuint64_t groups = ldn / 16, tiles = ((cuuint64_t)nbf * naux + oz::MT - 1) / oz::MT;
+        cuuint64_t dims[3] = {2 * oz::MT, groups, tiles * oz::SB};
+        cuuint64_t strides[2] = {16 * oz::MT, 16 * oz::MT * groups};
+        cuuint32_t box[3] = {2 * oz::MT, 8, 1};
+        DONOF_CHECK(make_tmap_u64_flat(ctx, &ma, job->oz_b, 3, dims, strides, box));
+    }
+    DONOF_CHECK(map_c5(job, nbf5, &mb));
+    oz::Params P = base_params(job, nbf5);
+    const int grid = shape_c5(ctx, P, (long long)nbf * naux);
+    prof_begin(ctx, st);
+    if (out) {
+        P.out = out;
+        DONOF_CHECK(launch_oz<oz::T1_F64>(ctx, st, ma, mb, P, grid));
+    } else {
+        P.t8 = job->tmp.as<int8_t>();
+        DONOF_CHECK(launch_oz<oz::T1_DIGITS>(ctx, st, ma, mb, P, grid));
+    }
+    prof_end(ctx, st);
+    return DONOF_OK;
+}
 
 }  // namespace
 
 bool ozaki_shape_ok(int nbf) { return nbf >= 1 && nbf <= 16384; }
 
-size_t ozaki_bytes(int nbf, int naux) {
-    return align256(slice_bytes(nbf, naux)) + sizeof(double) * (size_t)nbf * naux;
-}
+size_t ozaki_bytes(int nbf, int naux) { return job_layout(nbf, naux).bytes; }
 
 // Digit slices and row scales of the job's b (kept until ozaki_free).
 int ozaki_build(donof_job* job) {
@@ -494,16 +1142,20 @@ int ozaki_build(donof_job* job) {
         set_error(ctx, "the tensor-core FP64 transform needs nbf <= 16384 (got %d)", nbf);
         return DONOF_ERR_ARG;
     }
+    const JobLayout jl = job_layout(nbf, naux);
     void* buf = nullptr;
-    DONOF_CHECK(dev_alloc(ctx, &buf, ozaki_bytes(nbf, naux)));
+    DONOF_CHECK(dev_alloc(ctx, &buf, jl.bytes));
     int8_t* slices = static_cast<int8_t*>(buf);
-    double* sa = reinterpret_cast<double*>(static_cast<char*>(buf) + align256(slice_bytes(nbf, naux)));
+    double* ra = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.ra);
+    double* RL = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.rl);
+    unsigned long long* rn = reinterpret_cast<unsigned long long*>(RL + naux);
     cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaMemsetAsync(slices, 0, slice_bytes(nbf, naux), st);
+    cudaError_t e = cudaMemsetAsync(rn, 0, sizeof(unsigned long long) * (size_t)naux, st);
     if (e == cudaSuccess) {
-        oz::row_scale_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(job->b, nbf, (long long)naux, sa); count_launch();
-        oz::split_b_kernel<<<16 * ctx->sm_count, 256, 0, st>>>(job->b, sa, nbf, ldn_of(nbf), (long long)naux, slices);
+        oz::row_scale_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(job->b, nbf, (long long)naux, ra, rn); count_launch();
+        oz::split_b_kernel<<<16 * ctx->sm_count, 256, 0, st>>>(job->b, ra, nbf, ldn_of(nbf), (long long)naux, slices);
         count_launch();
+        oz::row_finish_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(nbf, (long long)naux, rn, RL, ra); count_launch();
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -513,7 +1165,6 @@ int ozaki_build(donof_job* job) {
         return DONOF_ERR_CUDA;
     }
     job->oz_b = buf;
-    job->oz_sa = sa;
     ++job->oz_gen;
     return DONOF_OK;
 }
@@ -523,57 +1174,104 @@ void ozaki_free(donof_job* job) {
     cudaStreamSynchronize(job->ctx->stream);
     dev_free(job->ctx, job->oz_b);
     job->oz_b = nullptr;
-    job->oz_sa = nullptr;
     job->oz_c.release(job->ctx);
     ++job->oz_gen;
 }
 
 // tmp_l = B_l C5 for every l (FP64 result, tmp[m + nbf*q + nbf*nbf5*l]).
 int t1_ozaki(donof_job* job, cudaStream_t st, const double* C, int nbf5, double* tmp) {
+    DONOF_CHECK(prep(job, st, C, nullptr, nullptr, nullptr, nbf5));
+    return t1(job, st, nbf5, tmp);
+}
+
+// T1 and T2: tmp's digit slices into job->tmp, b_pq into job->bpq.  n, cj12 and
+// ck12 (or null) are the coefficients of the W that y_ozaki will build.
+int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
+                     const double* ck12, int nbf5) {
     donof_ctx* ctx = job->ctx;
-    const int nbf = job->nbf, naux = job->naux, ldn = ldn_of(nbf);
-    const size_t cbytes = align256((size_t)oz::S * nbf5 * ldn);
-    DONOF_CHECK(job->oz_c.ensure(ctx, cbytes + sizeof(double) * (size_t)nbf5));
-    int8_t* c8 = job->oz_c.as<int8_t>();
-    double* sb = reinterpret_cast<double*>(job->oz_c.as<char>() + cbytes);
-    oz::split_c_kernel<<<nbf5, 256, 0, st>>>(C, nbf, nbf5, ldn, sb, c8); count_launch();
+    const int nbf = job->nbf, naux = job->naux;
+    DONOF_CHECK(job->tmp.ensure(ctx, (size_t)oz::SW * nbf * oz::KC * chunks_of(nbf5, naux)));
+    DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * nbf5 * naux));
+    DONOF_CHECK(prep(job, st, C, n, cj12, ck12, nbf5));
+    DONOF_CHECK(t1(job, st, nbf5, nullptr));
+    CUtensorMap ma, mb;
+    DONOF_CHECK(map_t8(job, nbf5, &ma));
+    DONOF_CHECK(map_c5(job, nbf5, &mb));
+    oz::Params P = base_params(job, nbf5);
+    const int grid = shape_c5(ctx, P, (long long)P.ldq * naux);
+    P.out = job->bpq.as<double>();
+    return launch_oz<oz::T2>(ctx, st, ma, mb, P, grid);
+}
+
+// W from job->bpq and Y = sum_l tmp_l W_l as FP64 partials (nbf x nbf5 each) in
+// job->part, after transforms_ozaki with the same coefficients.
+int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12, const double* ck12, int nbf5,
+            int nalpha, int nbeta, const double** ypart, int* nparts) {
+    donof_ctx* ctx = job->ctx;
+    const int nbf = job->nbf, naux = job->naux, ldq = ldq_of(nbf5), nch = chunks_of(nbf5, naux);
+    const size_t wbytes = (size_t)oz::SW * nbf5 * oz::KC * nch;
+    const JobLayout jl = job_layout(nbf, naux);
+    const bool in_job = wbytes <= jl.ra - jl.work;
+    const size_t o_tv = in_job ? 0 : align256(wbytes);
+    DONOF_CHECK(job->W.ensure(ctx, o_tv + sizeof(double) * (size_t)nbf5 * naux));
+    int8_t* w8 = in_job ? reinterpret_cast<int8_t*>(static_cast<char*>(job->oz_b) + jl.work) : job->W.as<int8_t>();
+    double* tv = reinterpret_cast<double*>(job->W.as<char>() + o_tv);
+    oz::Params P = base_params(job, nbf5);
+    const double* bpq = job->bpq.as<double>();
+    {
+        const dim3 grid((naux + oz::LB - 1) / oz::LB, (nbf5 + 31) / 32);
+        oz::diag_kernel<<<grid, 256, 0, st>>>(bpq, n, cj12, nbf5, naux, nalpha, nbeta, P.RL, P.CN, P.beta, tv, P.wmax);
+        count_launch();
+    }
+    {
+        const long long items = (long long)((nbf5 + 31) / 32 * 32) * nch * 8;
+        long long blocks = (items + 255) / 256;
+        if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
+        oz::w_digits_kernel<<<(int)blocks, 256, 0, st>>>(bpq, ck12, tv, nbf5, naux, ldq, nch, P.RL, P.CN, P.beta, P.wmax,
+                                                            w8);
+        count_launch();
+    }
     DONOF_CUDA(ctx, cudaGetLastError());
 
+    constexpr int stage = oz::SW * oz::BS_BYTES;
+    P.nrt = (nbf + oz::MT - 1) / oz::MT;
+    P.nct = (nbf5 + oz::QT - 1) / oz::QT;
+    P.nkc = nch;
+    P.k4_last = (int)(((long long)ldq * naux - (long long)(nch - 1) * oz::KC + 31) / 32);
+    P.ring_off = 2 * stage;
+    P.ring = (oz::DATA_BYTES - P.ring_off) / oz::A_BYTES;
+    if (P.ring > oz::RING_MAX) P.ring = oz::RING_MAX;
+    // The split of K: waves of units over the SMs, each unit a few chunks (about 3.5
+    // us each, and 2 us to fill and drain), and the partials written and summed by
+    // the tail.  A rule of the shape alone, so that a shape sums in one order.
+    const int tiles = P.nrt * P.nct;
+    double best = 0.0;
+    for (int s = 1; s <= P.nkc && s <= 1024; ++s) {
+        const int cpu = (P.nkc + s - 1) / s;
+        if (cpu > oz::KMAX_CHUNKS) continue;
+        const int used = (P.nkc + cpu - 1) / cpu;
+        const long long waves = ((long long)tiles * used + ctx->sm_count - 1) / ctx->sm_count;
+        const double cost = waves * (3.5 * cpu + 2.0) + used * ((double)nbf * nbf5 * 16.0 / 3e6);
+        if (best == 0.0 || cost < best) {
+            best = cost;
+            P.cpu = cpu;
+            P.nsplit = used;
+        }
+    }
+    if (best == 0.0) {  // more than 1024 units of the longest exact range
+        P.cpu = oz::KMAX_CHUNKS;
+        P.nsplit = (P.nkc + P.cpu - 1) / P.cpu;
+    }
+    DONOF_CHECK(job->part.ensure(ctx, sizeof(double) * (size_t)P.nsplit * nbf * nbf5));
+    P.out = job->part.as<double>();
     CUtensorMap ma, mb;
-    {
-        cuuint64_t dims[4] = {(cuuint64_t)nbf, (cuuint64_t)nbf, (cuuint64_t)oz::S, (cuuint64_t)naux};
-        cuuint64_t strides[3] = {(cuuint64_t)ldn, (cuuint64_t)ldn * nbf, (cuuint64_t)ldn * nbf * oz::S};
-        cuuint32_t box[4] = {oz::KC, oz::MT, 1, 1};
-        DONOF_CHECK(make_tmap_u8(ctx, &ma, job->oz_b, 4, dims, strides, box));
-    }
-    {
-        cuuint64_t dims[3] = {(cuuint64_t)nbf, (cuuint64_t)nbf5, (cuuint64_t)oz::S};
-        cuuint64_t strides[2] = {(cuuint64_t)ldn, (cuuint64_t)ldn * nbf5};
-        cuuint32_t box[3] = {oz::KC, oz::QT, oz::S};
-        DONOF_CHECK(make_tmap_u8(ctx, &mb, c8, 3, dims, strides, box));
-    }
-    oz::Params P{};
-    P.nbf = nbf; P.nbf5 = nbf5; P.naux = naux;
-    P.nmt = (nbf + oz::MT - 1) / oz::MT;
-    P.nkc = (nbf + oz::KC - 1) / oz::KC;
-    P.nqt = (nbf5 + oz::QT - 1) / oz::QT;
-    P.resident = P.nqt * P.nkc <= 2;
-    P.sa = job->oz_sa; P.sb = sb; P.tmp = tmp;
-    P.fail = ctx->fail_dev ? ctx->fail_dev + FAIL_MBAR : nullptr;
-    P.wait = sm100::wait_budget(ctx->wait_limit);
-    const long long units = (long long)naux * P.nmt;
+    DONOF_CHECK(map_t8(job, nbf5, &ma));
+    DONOF_CHECK(map_b(job, w8, nbf5, oz::SW, nch, &mb));
+    const long long units = (long long)tiles * P.nsplit;
     const int grid = (int)(units < ctx_ctas(ctx) ? units : ctx_ctas(ctx));
-    static std::atomic<unsigned long long> attr_mask{0};
-    const unsigned long long bit = 1ull << (ctx->device & 63);
-    if (!(attr_mask.load(std::memory_order_acquire) & bit)) {
-        DONOF_CUDA(ctx, cudaFuncSetAttribute(oz::ozaki_t1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             oz::SMEM_ALLOC));
-        attr_mask.fetch_or(bit, std::memory_order_acq_rel);
-    }
-    prof_begin(ctx, st);
-    oz::ozaki_t1_kernel<<<grid, oz::NTHREADS, oz::SMEM_ALLOC, st>>>(ma, mb, P); count_launch();
-    prof_end(ctx, st);
-    DONOF_CUDA(ctx, cudaGetLastError());
+    DONOF_CHECK(launch_oz<oz::YSUM>(ctx, st, ma, mb, P, grid));
+    *ypart = job->part.as<double>();
+    *nparts = P.nsplit;
     return DONOF_OK;
 }
 

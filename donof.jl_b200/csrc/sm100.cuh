@@ -109,6 +109,13 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46) | (2ull << 61);
 }
+// The same without swizzle: core matrices of 8 rows x 16 bytes (128 contiguous
+// bytes).  K-major operand: lbo between core matrices along K, sbo along M or N;
+// MN-major: sbo between core matrices along M or N, lbo along K.
+__device__ __forceinline__ uint64_t sdesc_flat(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
+           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
+}
 // instruction descriptor: bf16 x bf16 -> f32
 __host__ __device__ constexpr uint32_t idesc(int M, int N, int a_mn, int b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
@@ -134,6 +141,18 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t a, uint64_t b,
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(a), "l"(b), "r"(id), "r"(accum));
+}
+// One lane of a converged warp (the same one every time).  The branches of a
+// warp that is otherwise uniform keep their descriptors in uniform registers: an
+// MMA issued this way takes about half the issue slots of one behind lane == 0.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "elect.sync _|P, 0xffffffff;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}"
+        : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -177,6 +196,13 @@ __device__ __forceinline__ void tmem_issue16(uint32_t taddr, uint32_t (&r)[16]) 
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
+}
+// Store zeros to 16 TMEM columns of the warp's 32 lanes (valid after tmem_wait_st()).
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    const uint32_t z = 0;
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(z)
+        : "memory");
 }
 // Store zeros to 32 TMEM columns of the warp's 32 lanes (valid after tmem_wait_st()).
 __device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
