@@ -17,14 +17,15 @@ namespace donof {
 namespace {
 
 // Vs[i + n j] = V[i + n j] s_j,  VT[j + n i] = V[i + n j];  s_j = 1/sqrt(w_j), 0 for w_j < 0
-__global__ void gmsqrt_factors_kernel(const double* __restrict__ V, const double* __restrict__ w, int n,
+// (V's leading dimension is ldv, the others' n)
+__global__ void gmsqrt_factors_kernel(const double* __restrict__ V, const double* __restrict__ w, int n, int ldv,
                                       double* __restrict__ Vs, double* __restrict__ VT) {
     const long long total = (long long)n * n;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(idx % n), j = (int)(idx / n);
         const double s = (w[j] < 0.0) ? 0.0 : 1.0 / sqrt(w[j]);
-        const double v = V[idx];
+        const double v = V[i + (long long)ldv * j];
         Vs[idx] = v * s;
         VT[j + (long long)n * i] = v;
     }
@@ -57,6 +58,7 @@ struct DeviceScratch {
 int iaux_f64(donof_ctx* ctx, cudaStream_t st, const double* G_host, const double* I_host, int nbf, int naux,
              double* b, DevBuf* part) {
     const size_t nn = (size_t)nbf * nbf, na2 = (size_t)naux * naux;
+    const int npad = eigh_padded(naux);
     DeviceScratch s(ctx);
     double *dI = nullptr, *dG = nullptr, *dw = nullptr, *dVs = nullptr, *dVT = nullptr, *dGm = nullptr,
            *dA = nullptr, *dV = nullptr;
@@ -67,17 +69,18 @@ int iaux_f64(donof_ctx* ctx, cudaStream_t st, const double* G_host, const double
     DONOF_CHECK(s.alloc(&dVs, na2));
     DONOF_CHECK(s.alloc(&dVT, na2));
     DONOF_CHECK(s.alloc(&dGm, na2));
-    DONOF_CHECK(s.alloc(&dA, na2));
-    DONOF_CHECK(s.alloc(&dV, na2));
+    DONOF_CHECK(s.alloc(&dA, (size_t)npad * npad));
+    DONOF_CHECK(s.alloc(&dV, (size_t)npad * npad));
     DONOF_CHECK(s.alloc(&escr, eigh_scratch_bytes(naux)));
-    DONOF_CUDA(ctx, cudaMemcpyAsync(dI, I_host, sizeof(double) * nn * naux, cudaMemcpyHostToDevice, st));
     DONOF_CUDA(ctx, cudaMemcpyAsync(dG, G_host, sizeof(double) * na2, cudaMemcpyHostToDevice, st));
     // eigen-decomposition of Symmetric(G) (its upper triangle)
     DONOF_CHECK(eigh_jacobi(ctx, st, dG, naux, dA, dV, dw, escr));
+    DONOF_CUDA(ctx, cudaMemcpyAsync(dI, I_host, sizeof(double) * nn * naux, cudaMemcpyHostToDevice, st));
+    DONOF_CHECK(eigh_finish(ctx, st, escr));
     {
         long long blocks = ((long long)na2 + 255) / 256;
         if (blocks > 8LL * ctx->sm_count) blocks = 8LL * ctx->sm_count;
-        gmsqrt_factors_kernel<<<(int)blocks, 256, 0, st>>>(dV, dw, naux, dVs, dVT); count_launch();
+        gmsqrt_factors_kernel<<<(int)blocks, 256, 0, st>>>(dV, dw, naux, npad, dVs, dVT); count_launch();
         DONOF_CUDA(ctx, cudaGetLastError());
     }
     // G^{-1/2} = Vs V^T (A: Vs, M-contiguous; B: V^T stored K-contiguous)

@@ -75,11 +75,14 @@ int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double
                   double* E);
 
 // Eigenvalues w and eigenvectors V (columns) of Symmetric(G) on the device by
-// the parallel cyclic Jacobi method (eigh.cu); A: n x n scratch, scratch:
-// eigh_scratch_bytes(n).  Synchronises the stream.
+// the parallel block Jacobi method (eigh.cu): A and V hold N x N with N =
+// eigh_padded(n) (V's leading dimension is N), scratch eigh_scratch_bytes(n).
+// eigh_jacobi enqueues; eigh_finish synchronises the stream and reports.
+int eigh_padded(int n);
 size_t eigh_scratch_bytes(int n);
 int eigh_jacobi(donof_ctx* ctx, cudaStream_t st, const double* G, int n, double* A, double* V, double* w,
                 void* scratch);
+int eigh_finish(donof_ctx* ctx, cudaStream_t st, const void* scratch);
 
 // b = I G^{-1/2} on the device from host G (naux x naux) and I (nbf x nbf x naux)
 // (iaux.cu); part is scratch for the products.
@@ -107,8 +110,6 @@ int make_tmap_u64_flat(donof_ctx* ctx, CUtensorMap* map, const void* base, int r
                        const cuuint64_t* strides_bytes, const cuuint32_t* box);
 int make_tmap_bf16(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
                    const cuuint64_t* strides_bytes, const cuuint32_t* box);
-int make_tmap_u8(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
-                 const cuuint64_t* strides_bytes, const cuuint32_t* box);
 
 // FP64 pipelines (lagrange.cu)
 int transforms_f64(donof_job* job, cudaStream_t st, const double* C, int nbf5);

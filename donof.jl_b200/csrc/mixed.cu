@@ -646,8 +646,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 // Tensor map with zero fill outside the tensor (no interleave): bf16 with 128-byte
 // swizzle for the mixed kernels of this file and mixed_general.cu; for the digit
-// slices of ozaki.cu 8-bit with 128-byte swizzle, and 64-bit without swizzle
-// (16-byte core-matrix rows, two elements each).
+// slices of ozaki.cu 64-bit without swizzle (16-byte core-matrix rows, two elements
+// each).
 static int make_tmap(donof_ctx* ctx, CUtensorMap* map, CUtensorMapDataType dtype, const void* base, int rank,
                      const cuuint64_t* dims, const cuuint64_t* strides_bytes, const cuuint32_t* box,
                      CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
@@ -655,11 +655,6 @@ static int make_tmap(donof_ctx* ctx, CUtensorMap* map, CUtensorMapDataType dtype
 int make_tmap_bf16(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
              const cuuint64_t* strides_bytes, const cuuint32_t* box) {
     return make_tmap(ctx, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, dims, strides_bytes, box);
-}
-
-int make_tmap_u8(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
-                 const cuuint64_t* strides_bytes, const cuuint32_t* box) {
-    return make_tmap(ctx, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, rank, dims, strides_bytes, box);
 }
 
 int make_tmap_u64_flat(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
