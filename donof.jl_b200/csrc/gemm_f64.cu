@@ -451,7 +451,8 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ part, long long 
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
          i += (long long)gridDim.x * blockDim.x) {
         double s = 0.0;
-        for (int k = 0; k < splits; ++k) s += part[i + k * stride];
+#pragma unroll 8
+        for (int k = 0; k < splits; ++k) s += part[i + k * stride];  // in order; eight loads in flight
         out[i] = (beta != 0.0) ? s + beta * out[i] : s;
     }
 }

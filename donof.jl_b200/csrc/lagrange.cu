@@ -17,6 +17,7 @@
 
 #include <mutex>
 
+#include "jk.cuh"
 #include "kernels.cuh"
 #include "wbuild.cuh"
 
@@ -159,26 +160,6 @@ __global__ void e_elec_kernel(const double* __restrict__ elag, const double* __r
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (threadIdx.x == 0) *E = s;
     }
-}
-
-// J/K partial sums over a chunk of aux indices; thread per (p, q).
-__global__ void jk_partial_kernel(const double* __restrict__ bpq, int nbf5, int naux, int lchunk,
-                                  double* __restrict__ part) {
-    const long long n55 = (long long)nbf5 * nbf5;
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (idx >= n55) return;
-    const int p = (int)(idx % nbf5), q = (int)(idx / nbf5);
-    const int l0 = c * lchunk, l1 = min(naux, l0 + lchunk);
-    double sj = 0.0, sk = 0.0;
-    for (int l = l0; l < l1; ++l) {
-        const double* B = bpq + n55 * l;
-        const double v = B[idx];
-        sj += B[(long long)p * (nbf5 + 1)] * B[(long long)q * (nbf5 + 1)];
-        sk += v * v;
-    }
-    part[(long long)c * 2 * n55 + idx] = sj;
-    part[(long long)c * 2 * n55 + n55 + idx] = sk;
 }
 
 // H_core[i] = sum_m C[m,i] (H C5)[m,i]; one warp per i.
@@ -325,17 +306,11 @@ int jkh_mo_f64(donof_job* job, cudaStream_t st, const double* C, const double* H
     const int nbf = job->nbf, naux = job->naux;
     DONOF_CHECK(transforms_f64(job, st, C, nbf5));
     const long long n55 = (long long)nbf5 * nbf5;
-    // chunk the aux index so that about 2 CTAs per SM are busy
-    const int xblocks = (int)((n55 + 255) / 256);
-    int chunks = (2 * ctx->sm_count + xblocks - 1) / xblocks;
-    if (chunks > naux) chunks = naux;
-    if (chunks < 1) chunks = 1;
-    const int lchunk = (naux + chunks - 1) / chunks;
-    chunks = (naux + lchunk - 1) / lchunk;
+    const int lchunk = jk::chunk(nbf5, naux, ctx->sm_count);
+    const int chunks = (naux + lchunk - 1) / lchunk;
     DONOF_CHECK(job->part.ensure(ctx, sizeof(double) * (size_t)chunks * 2 * n55));
     double* part = job->part.as<double>();
-    jk_partial_kernel<<<dim3(xblocks, chunks), 256, 0, st>>>(job->bpq.as<double>(), nbf5, naux, lchunk,
-                                                             part); count_launch();
+    jk::launch_partial(st, job->bpq.as<double>(), nbf5, naux, lchunk, part);
     DONOF_CUDA(ctx, cudaGetLastError());
     DONOF_CHECK(splitk_reduce(ctx, st, part, 2 * n55, chunks, n55, J, 0.0));
     DONOF_CHECK(splitk_reduce(ctx, st, part + n55, 2 * n55, chunks, n55, K, 0.0));

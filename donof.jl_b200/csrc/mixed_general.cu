@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "jk.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"
 
@@ -352,65 +353,101 @@ __global__ void mg_prep_kernel(const double* __restrict__ C, int nbf, int nbf5, 
 // contiguous q: the K-major A operand of Y):
 //   W[q, b] = delta_qb (n'_b d_b + sum_q' cj12[b, q'] d_q') - ck12[b, q] b_pq[q, b]
 // with d_q = b_pq[q, q] and n'_b = n_b for b < nbeta or b >= nalpha (0 when
-// nbeta = 0); b_pq is symmetric, so its row b is read as column b.  mg_wdiag
-// forms the diagonal terms (one thread per (b, l)), mg_w the elements (one
-// thread per element, reads and writes along q).
-__global__ void mg_wdiag_kernel(const float* __restrict__ bpq, const float* __restrict__ n32,
-                                const float* __restrict__ cj32, int nbf5, int naux, int nalpha, int nbeta,
-                                float* __restrict__ tv) {
-    const long long n55 = (long long)nbf5 * nbf5, total = (long long)nbf5 * naux;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(i % nbf5);
-        const float* B = bpq + n55 * (i / nbf5);
-        float s = 0.f;
-        for (int q = 0; q < nbf5; ++q) s += cj32[b + (long long)nbf5 * q] * B[(long long)q * (nbf5 + 1)];
-        const bool dj = (nbeta > 0) && (b < nbeta || b >= nalpha);
-        tv[i] = (dj ? n32[b] * B[(long long)b * (nbf5 + 1)] : 0.f) + s;
-    }
-}
+// nbeta = 0); b_pq is symmetric, so its row b is read as column b.
+// mg_wdiag forms the diagonal terms: a block takes WL aux indices, their diagonals
+// staged in shared memory, a thread all of them for its b (a cj12 element serves WL
+// products, each sum still in the order of q).  One thread per (b, l), reading the
+// diagonals at a stride of nbf5 + 1, took 58 us at nbf5 = 198, naux = 974.
+constexpr int WL = 8;
+constexpr int WQ = 512;  // diagonal elements staged at a time
 
-__global__ void mg_w_kernel(const float* __restrict__ bpq, const float* __restrict__ ckT,
-                            const float* __restrict__ tv, int nbf5, int ldq, int naux,
-                            __nv_bfloat16* __restrict__ w_hi, __nv_bfloat16* __restrict__ w_lo) {
-    const long long n55 = (long long)nbf5 * nbf5, total = (long long)ldq * nbf5 * naux;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i % ldq);
-        const long long r = i / ldq;  // b + nbf5 l
-        const int b = (int)(r % nbf5);
-        const long long l = r / nbf5;
-        float v = 0.f;
-        if (q < nbf5) {
-            v = -ckT[q + (long long)nbf5 * b] * bpq[q + (long long)nbf5 * b + n55 * l];
-            if (q == b) v += tv[r];
-        }
-        __nv_bfloat16 h, lo;
-        split_bf16(v, h, lo);
-        w_hi[i] = h;
-        w_lo[i] = lo;
-    }
-}
-
-// J and K partial sums over an aux chunk from FP32 b_pq, accumulated in FP64:
-// part[c][0][p + nbf5 q] = sum_l d_p d_q,  part[c][1][p + nbf5 q] = sum_l b_pq^2
-__global__ void mg_jk_partial_kernel(const float* __restrict__ bpq, int nbf5, int naux, int lchunk,
-                                     double* __restrict__ part) {
+__global__ void __launch_bounds__(256) mg_wdiag_kernel(const float* __restrict__ bpq, const float* __restrict__ n32,
+                                                       const float* __restrict__ cj32, int nbf5, int naux, int nalpha,
+                                                       int nbeta, float* __restrict__ tv) {
+    __shared__ __align__(16) float sd[WQ][WL];
     const long long n55 = (long long)nbf5 * nbf5;
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (idx >= n55) return;
-    const int p = (int)(idx % nbf5), q = (int)(idx / nbf5);
-    const int l0 = c * lchunk, l1 = min(naux, l0 + lchunk);
-    double sj = 0.0, sk = 0.0;
-    for (int l = l0; l < l1; ++l) {
-        const float* B = bpq + n55 * l;
-        const double v = B[idx];
-        sj += (double)B[(long long)p * (nbf5 + 1)] * (double)B[(long long)q * (nbf5 + 1)];
-        sk += v * v;
+    const int l0 = blockIdx.x * WL;
+    for (int b0 = 0; b0 < nbf5; b0 += blockDim.x) {
+        const int b = b0 + threadIdx.x;
+        float s[WL];
+#pragma unroll
+        for (int k = 0; k < WL; ++k) s[k] = 0.f;
+        for (int p0 = 0; p0 < nbf5; p0 += WQ) {
+            const int np = min(WQ, nbf5 - p0);
+            __syncthreads();
+            jk::stage_diagonals<8>(bpq + n55 * l0, nbf5, p0, np, min(WL, naux - l0), &sd[0][0], 1, WL);
+            __syncthreads();
+            if (b < nbf5) {
+#pragma unroll 16
+                for (int q = 0; q < np; ++q) {
+                    const float c = cj32[b + (long long)nbf5 * (p0 + q)];
+                    const float4 x = *reinterpret_cast<const float4*>(sd[q]), y = *reinterpret_cast<const float4*>(sd[q] + 4);
+                    const float d[WL] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for (int k = 0; k < WL; ++k) s[k] += c * d[k];
+                }
+            }
+        }
+        if (b < nbf5) {
+            const bool dj = (nbeta > 0) && (b < nbeta || b >= nalpha);
+            const float nb = dj ? n32[b] : 0.f;
+#pragma unroll
+            for (int k = 0; k < WL; ++k)
+                if (l0 + k < naux) {
+                    const float d = bpq[n55 * (l0 + k) + (long long)b * (nbf5 + 1)];
+                    tv[b + (long long)nbf5 * (l0 + k)] = (dj ? nb * d : 0.f) + s[k];
+                }
+        }
     }
-    part[(long long)c * 2 * n55 + idx] = sj;
-    part[(long long)c * 2 * n55 + n55 + idx] = sk;
+}
+
+// mg_w forms the elements: a warp per row (b, l), lanes on pairs of q, the loads of
+// 256 q in flight together.  Element by element with 64-bit index divisions it took
+// 166 us at nbf5 = 198, naux = 974 for 315 MB.
+__global__ void __launch_bounds__(256) mg_w_kernel(const float* __restrict__ bpq, const float* __restrict__ ckT,
+                                                   const float* __restrict__ tv, int nbf5, int ldq, int naux,
+                                                   __nv_bfloat16* __restrict__ w_hi, __nv_bfloat16* __restrict__ w_lo) {
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)nbf5 * naux, stride = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long r = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += stride) {
+        const int b = (int)(r % nbf5);
+        const float* B = bpq + (long long)nbf5 * r;  // row b of b_pq^l
+        const float* ck = ckT + (long long)nbf5 * b;
+        const float t = tv[r];
+        __nv_bfloat16 *hi = w_hi + (long long)ldq * r, *lo = w_lo + (long long)ldq * r;
+        for (int q0 = 0; q0 < ldq; q0 += 256) {
+            float x[4][2], c[4][2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int q = q0 + 64 * k + 2 * lane + e;
+                    const bool in = q < nbf5;
+                    x[k][e] = in ? B[q] : 0.f;
+                    c[k][e] = in ? ck[q] : 0.f;
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = q0 + 64 * k + 2 * lane;
+                if (q >= ldq) break;  // ldq is even
+                __nv_bfloat162 h, l;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float v = 0.f;
+                    if (q + e < nbf5) {
+                        v = -c[k][e] * x[k][e];
+                        if (q + e == b) v += t;
+                    }
+                    __nv_bfloat16 vh, vl;
+                    split_bf16(v, vh, vl);
+                    if (e == 0) { h.x = vh; l.x = vl; }
+                    else { h.y = vh; l.y = vl; }
+                }
+                *reinterpret_cast<__nv_bfloat162*>(hi + q) = h;
+                *reinterpret_cast<__nv_bfloat162*>(lo + q) = l;
+            }
+        }
+    }
 }
 
 // tmp[m + nbf q + nbf nbf5 l] = tmpQ_hi + tmpQ_lo (FP32, for checks of T1)
@@ -589,12 +626,10 @@ int lagrange2_mixed_general(donof_job* job, cudaStream_t st, const double* C, co
     DONOF_CHECK(gen_prepare(job, st, C, n, cj12, ck12, nbf5, true, &S));
     DONOF_CHECK(gen_transforms(job, st, nbf5, S));
     {
-        const long long nd = (long long)nbf5 * naux, nw = (long long)S.ldq * nbf5 * naux;
-        long long blocks = (nd + 255) / 256;
-        if (blocks > 8LL * ctx->sm_count) blocks = 8LL * ctx->sm_count;
-        mg::mg_wdiag_kernel<<<(int)blocks, 256, 0, st>>>(S.bpq, S.n32, S.cj32, nbf5, naux, nalpha, nbeta,
-                                                         S.tv); count_launch();
-        blocks = (nw + 255) / 256;
+        const int threads = nbf5 >= 256 ? 256 : (nbf5 + 31) / 32 * 32;
+        mg::mg_wdiag_kernel<<<(naux + mg::WL - 1) / mg::WL, threads, 0, st>>>(S.bpq, S.n32, S.cj32, nbf5, naux,
+                                                                             nalpha, nbeta, S.tv); count_launch();
+        long long blocks = ((long long)nbf5 * naux + 7) / 8;
         if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
         mg::mg_w_kernel<<<(int)blocks, 256, 0, st>>>(S.bpq, S.ckT, S.tv, nbf5, S.ldq, naux, S.w_hi,
                                                      S.w_lo); count_launch();
@@ -646,15 +681,11 @@ int jkh_mo_mixed_general(donof_job* job, cudaStream_t st, const double* C, const
     DONOF_CHECK(gen_prepare(job, st, C, nullptr, nullptr, nullptr, nbf5, false, &S));
     DONOF_CHECK(gen_transforms(job, st, nbf5, S));
     const long long n55 = (long long)nbf5 * nbf5;
-    const int xblocks = (int)((n55 + 255) / 256);
-    int chunks = (2 * ctx->sm_count + xblocks - 1) / xblocks;
-    if (chunks > naux) chunks = naux;
-    if (chunks < 1) chunks = 1;
-    const int lchunk = (naux + chunks - 1) / chunks;
-    chunks = (naux + lchunk - 1) / lchunk;
+    const int lchunk = jk::chunk(nbf5, naux, ctx->sm_count);
+    const int chunks = (naux + lchunk - 1) / lchunk;
     DONOF_CHECK(job->part.ensure(ctx, sizeof(double) * (size_t)chunks * 2 * n55));
     double* part = job->part.as<double>();
-    mg::mg_jk_partial_kernel<<<dim3(xblocks, chunks), 256, 0, st>>>(S.bpq, nbf5, naux, lchunk, part); count_launch();
+    jk::launch_partial(st, S.bpq, nbf5, naux, lchunk, part);
     DONOF_CUDA(ctx, cudaGetLastError());
     DONOF_CHECK(splitk_reduce(ctx, st, part, 2 * n55, chunks, n55, J, 0.0));
     DONOF_CHECK(splitk_reduce(ctx, st, part + n55, 2 * n55, chunks, n55, K, 0.0));

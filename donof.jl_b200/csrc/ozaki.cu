@@ -129,6 +129,7 @@ struct Params {
     unsigned* wmax;            // [0] of |RL CN b_pq|, [1] of |RL CN t| / beta: high words of the largest value
     int8_t* t8;                // tmp's slices (see the layout above t8_at)
     double* out;               // FP64 output
+    double* diag;              // T2: b_qq^l at q + nbf5 l
     int* fail;                 // the context's failure word for mbarrier waits
     long long wait;            // cycle budget of every bounded wait (drains excepted)
 };
@@ -639,6 +640,12 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                     v[k] = v[k] * rs * P.sb2[q0 + k];  // b_pq (columns at and beyond nbf5: sb2 = 0)
                     if (in) top = max(top, (unsigned)__double2hiint(v[k] * rs) & 0x7fffffffu);
                 }
+                if (in && x >= q0 && x < q0 + NC) {
+                    double t = 0.0;
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) t = q0 + k == x ? v[k] : t;
+                    P.diag[x + (size_t)P.nbf5 * l] = t;
+                }
                 double* dst = P.out + ((size_t)P.nbf5 * l + x) * P.nbf5 + q0;
                 if (in && q0 + NC <= P.nbf5 && (P.nbf5 & 3) == 0) {
 #pragma unroll
@@ -846,38 +853,35 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
 // ---------------------------------------------------------------- W
 // tv[b + nbf5 l] = n'_b d_b^l + sum_q cj12[b, q] d_q^l with d_q^l = b_pq^l[q, q]
 // (lagrange.cu), and the largest |RL CN tv| / beta.  A block takes 32 b of LB aux
-// indices: the diagonals staged in shared memory a panel of DQ at a time, each of
+// indices: the diagonals (D, written by T2) staged in shared memory a panel of DQ at a time, each of
 // its eight warps on an eighth of the panel's q (one cj12 element, read along b,
 // serves LB products), the eight partial sums added in a fixed order.
 constexpr int LB = 8;
 constexpr int DQ = 256;
 
-__global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ bpq, const double* __restrict__ n,
+__global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ D, const double* __restrict__ n,
                                                    const double* __restrict__ cj12, int nbf5, int naux, int nalpha,
                                                    int nbeta, const double* __restrict__ RL,
                                                    const double* __restrict__ CN, const double* __restrict__ beta,
                                                    double* __restrict__ tv, unsigned* __restrict__ wmax) {
-    __shared__ double sd[DQ * LB];       // [q][LB]
+    __shared__ double sd[LB][DQ];
     __shared__ double part[8][LB][32];   // [warp][l][b]
     const int l0 = blockIdx.x * LB, b = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
-    const long long n55 = (long long)nbf5 * nbf5;
     double s[LB];
 #pragma unroll
     for (int k = 0; k < LB; ++k) s[k] = 0.0;
     for (int p0 = 0; p0 < nbf5; p0 += DQ) {
         const int np = min(DQ, nbf5 - p0);
         __syncthreads();
-        for (int i = threadIdx.x; i < LB * np; i += blockDim.x) {
-            const int k = i / np, q = i - k * np;
-            sd[q * LB + k] = l0 + k < naux ? bpq[n55 * (l0 + k) + (long long)(p0 + q) * (nbf5 + 1)] : 0.0;
-        }
+        if (l0 + warp < naux)  // warp k stages aux index l0 + k
+            for (int q = threadIdx.x & 31; q < np; q += 32) sd[warp][q] = D[(size_t)nbf5 * (l0 + warp) + p0 + q];
         __syncthreads();
         if (b < nbf5) {
-#pragma unroll 4
+#pragma unroll 8
             for (int q = warp; q < np; q += 8) {
                 const double c = cj12[b + (long long)nbf5 * (p0 + q)];
 #pragma unroll
-                for (int k = 0; k < LB; ++k) s[k] = fma(c, sd[q * LB + k], s[k]);
+                for (int k = 0; k < LB; ++k) s[k] = fma(c, sd[k][q], s[k]);
             }
         }
     }
@@ -891,7 +895,7 @@ __global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ bp
 #pragma unroll
         for (int w = 0; w < 8; ++w) t += part[w][warp][threadIdx.x & 31];
         const bool dj = (nbeta > 0) && (b < nbeta || b >= nalpha);
-        if (dj) t = fma(n[b], bpq[n55 * l + (long long)b * (nbf5 + 1)], t);
+        if (dj) t = fma(n[b], D[(size_t)nbf5 * l + b], t);
         tv[b + (long long)nbf5 * l] = t;
         const double be = beta[b];
         top = (unsigned)__double2hiint(RL[l] * t * (be == 0.0 ? 0.0 : CN[b] / be)) & 0x7fffffffu;
@@ -1191,7 +1195,8 @@ int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const dou
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
     DONOF_CHECK(job->tmp.ensure(ctx, (size_t)oz::SW * nbf * oz::KC * chunks_of(nbf5, naux)));
-    DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * nbf5 * naux));
+    // b_pq, and its diagonals again behind it
+    DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * (nbf5 + 1) * naux));
     DONOF_CHECK(prep(job, st, C, n, cj12, ck12, nbf5));
     DONOF_CHECK(t1(job, st, nbf5, nullptr));
     CUtensorMap ma, mb;
@@ -1200,6 +1205,7 @@ int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const dou
     oz::Params P = base_params(job, nbf5);
     const int grid = shape_c5(ctx, P, (long long)P.ldq * naux);
     P.out = job->bpq.as<double>();
+    P.diag = P.out + (size_t)nbf5 * nbf5 * naux;
     return launch_oz<oz::T2>(ctx, st, ma, mb, P, grid);
 }
 
@@ -1220,7 +1226,7 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
     const double* bpq = job->bpq.as<double>();
     {
         const dim3 grid((naux + oz::LB - 1) / oz::LB, (nbf5 + 31) / 32);
-        oz::diag_kernel<<<grid, 256, 0, st>>>(bpq, n, cj12, nbf5, naux, nalpha, nbeta, P.RL, P.CN, P.beta, tv, P.wmax);
+        oz::diag_kernel<<<grid, 256, 0, st>>>(bpq + (size_t)nbf5 * nbf5 * naux, n, cj12, nbf5, naux, nalpha, nbeta, P.RL, P.CN, P.beta, tv, P.wmax);
         count_launch();
     }
     {
