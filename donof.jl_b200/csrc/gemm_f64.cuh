@@ -141,9 +141,9 @@ struct GemmF64Cfg {
 // four steps that a kernel can interleave across tiles: init (operands,
 // extents, gates), prologue (the first STAGES - 1 cp.async stages, one commit
 // group each), mainloop (acc += A B over the tile's K range) and epilogue
-// (alpha, beta, column-major store).  gemm_f64_kernel runs them in order for
-// its one tile; the grouped persistent kernel issues the next tile's prologue
-// before the current tile's epilogue.  Both use the same staging and MMA order,
+// (alpha, beta, column-major store).  gemm_f64_kernel and the grouped kernel run
+// them in order for one tile; the persistent kernel issues the next tile's prologue
+// before the current tile's epilogue.  All use the same staging and MMA order,
 // so they write identical results.
 template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK, bool BKM, bool VEC>
 struct GemmTileF64 {
@@ -157,7 +157,8 @@ struct GemmTileF64 {
     double* Cout;
     long long lda, ldb, ldc;
     double alpha, beta;
-    int M, N, m0, n0, kbeg, kend, nk;
+    const double *srcA, *srcB;  // this thread's first copy of the next stage
+    int M, N, m0, n0, kend, nk, kload;
     bool use_beta, skip;
 
     __device__ __forceinline__ void init(const GemmF64Args& p, int bx, int by, int bz) {
@@ -165,14 +166,19 @@ struct GemmTileF64 {
         const int split = bz % p.splits;
         m0 = bx * BM;
         n0 = by * BN;
-        kbeg = split * p.kchunk;
+        const int kbeg = split * p.kchunk;
         kend = min(p.K, kbeg + p.kchunk);
+        kload = kbeg;
         nk = (kend > kbeg) ? (kend - kbeg + BK - 1) / BK : 0;
         A = p.A + (long long)z * p.strideA;
         B = (p.B_ptr != nullptr ? *p.B_ptr : p.B) + (long long)z * p.strideB;
         Cout = p.C + (long long)z * p.strideC + (p.splits > 1 ? (long long)split * p.strideSplit : 0LL);
         lda = p.lda; ldb = p.ldb; ldc = p.ldc;
         M = p.M; N = p.N;
+        srcA = AK ? A + (m0 + CopyA::line()) * lda + kbeg + CopyA::fast()
+                  : A + m0 + CopyA::fast() + (kbeg + CopyA::line()) * lda;
+        srcB = BKM ? B + (n0 + CopyB::line()) * ldb + kbeg + CopyB::fast()
+                   : B + n0 + CopyB::fast() + (kbeg + CopyB::line()) * ldb;
         alpha = p.alpha; beta = p.beta;
         use_beta = (p.splits == 1) && (p.beta != 0.0);
         skip = (p.skip_le != nullptr && *p.skip_le <= p.skip_level) || (p.skip_nz != nullptr && *p.skip_nz != 0);
@@ -183,61 +189,56 @@ struct GemmTileF64 {
         return smem + (size_t)s * Cfg::STAGE_ELEMS + Cfg::A_ELEMS;
     }
 
-    __device__ __forceinline__ void load(double* smem, int stage, int k0) const {
-        const int tid = threadIdx.x;
-        double* as = As(smem, stage);
-        double* bs = Bs(smem, stage);
-        // ---- A tile: BM x BK
-        if constexpr (AK) {
-            constexpr int CPR = BK / Cfg::VW;  // copies per row
-            for (int c = tid; c < BM * CPR; c += Cfg::THREADS) {
-                const int i = c / CPR, kk = (c % CPR) * Cfg::VW;
-                const int gi = m0 + i, gk = k0 + kk;
-                const bool ok = (gi < M) && (gk < kend);
-                const double* src = ok ? (A + (long long)gi * lda + gk) : A;
-                gemm_detail::cp_async<8 * Cfg::VW>(as + i * Cfg::SA + kk, src, ok);
-            }
-        } else {
-            constexpr int CPR = BM / Cfg::VW;
-            for (int c = tid; c < BK * CPR; c += Cfg::THREADS) {
-                const int kk = c / CPR, i = (c % CPR) * Cfg::VW;
-                const int gi = m0 + i, gk = k0 + kk;
-                const bool ok = (gi < M) && (gk < kend);
-                const double* src = ok ? (A + gi + (long long)gk * lda) : A;
-                gemm_detail::cp_async<8 * Cfg::VW>(as + kk * Cfg::SA + i, src, ok);
-            }
-        }
-        // ---- B tile: BK x BN
-        if constexpr (BKM) {
-            constexpr int CPR = BK / Cfg::VW;
-            for (int c = tid; c < BN * CPR; c += Cfg::THREADS) {
-                const int j = c / CPR, kk = (c % CPR) * Cfg::VW;
-                const int gj = n0 + j, gk = k0 + kk;
-                const bool ok = (gj < N) && (gk < kend);
-                const double* src = ok ? (B + gk + (long long)gj * ldb) : B;
-                gemm_detail::cp_async<8 * Cfg::VW>(bs + j * Cfg::SB + kk, src, ok);
-            }
-        } else {
-            constexpr int CPR = BN / Cfg::VW;
-            for (int c = tid; c < BK * CPR; c += Cfg::THREADS) {
-                const int kk = c / CPR, j = (c % CPR) * Cfg::VW;
-                const int gj = n0 + j, gk = k0 + kk;
-                const bool ok = (gj < N) && (gk < kend);
-                const double* src = ok ? (B + (long long)gk * ldb + gj) : B;
-                gemm_detail::cp_async<8 * Cfg::VW>(bs + kk * Cfg::SB + j, src, ok);
+    // A thread's copies of a stage: it keeps its place along the contiguous direction
+    // (Copier::fast) and steps across the lines (Copier::line), so a copy is a pointer
+    // addition and a bound on one index; the pointers move on by a stage per load.
+    // (With the indices and 64-bit offsets formed per copy, integer work was the
+    // busiest pipe of the 8-byte staging: 37% against 35% of the FP64 MMA.)
+    template <int LINES, int WIDTH>
+    struct Copier {
+        static constexpr int PER = WIDTH / Cfg::VW;          // copies per line
+        static constexpr int STEP = Cfg::THREADS / PER;      // lines per pass
+        static constexpr int PASSES = (LINES + STEP - 1) / STEP;
+        static_assert(Cfg::THREADS % PER == 0, "whole lines per pass");
+        static __device__ __forceinline__ int fast() { return (int)(threadIdx.x % PER) * Cfg::VW; }
+        static __device__ __forceinline__ int line() { return (int)(threadIdx.x / PER); }
+        // copies into dst (line stride ds); a line or a place beyond its limit is zero-filled
+        static __device__ __forceinline__ void run(double* dst, int ds, const double* src, long long ls, int lines_in,
+                                                   bool fast_in, const double* safe) {
+            double* d = dst + line() * ds + fast();
+#pragma unroll
+            for (int j = 0; j < PASSES; ++j) {
+                if (LINES % STEP != 0 && line() + j * STEP >= LINES) break;
+                const bool ok = fast_in && line() + j * STEP < lines_in;
+                gemm_detail::cp_async<8 * Cfg::VW>(d + j * STEP * ds, ok ? src : safe, ok);
+                src += STEP * ls;
             }
         }
+    };
+    using CopyA = Copier<AK ? BM : BK, AK ? BK : BM>;
+    using CopyB = Copier<BKM ? BN : BK, BKM ? BK : BN>;
+
+    // The stage of the next BK of K (kload), into ring slot `stage`.
+    __device__ __forceinline__ void load(double* smem, int stage) {
+        const int kleft = kend - kload;
+        CopyA::run(As(smem, stage), Cfg::SA, srcA, lda, AK ? M - m0 : kleft,
+                   CopyA::fast() < (AK ? kleft : M - m0), A);
+        CopyB::run(Bs(smem, stage), Cfg::SB, srcB, ldb, BKM ? N - n0 : kleft,
+                   CopyB::fast() < (BKM ? kleft : N - n0), B);
+        srcA += AK ? (long long)BK : BK * lda;
+        srcB += BKM ? (long long)BK : BK * ldb;
+        kload += BK;
     }
 
-    __device__ __forceinline__ void prologue(double* smem) const {
+    __device__ __forceinline__ void prologue(double* smem) {
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s) {
-            if (s < nk) load(smem, s, kbeg + s * BK);
+            if (s < nk) load(smem, s);
             gemm_detail::cp_async_commit();
         }
     }
 
-    __device__ __forceinline__ void mainloop(double* smem, Acc& acc) const {
+    __device__ __forceinline__ void mainloop(double* smem, Acc& acc) {
         const int lane = threadIdx.x & 31;
         const int warp = threadIdx.x >> 5;
         const int g = lane >> 2;  // groupID
@@ -255,7 +256,7 @@ struct GemmTileF64 {
             __syncthreads();
             {
                 const int nt = kt + STAGES - 1;
-                if (nt < nk) load(smem, nt % STAGES, kbeg + nt * BK);
+                if (nt < nk) load(smem, nt % STAGES);
                 gemm_detail::cp_async_commit();
             }
             const double* as = As(smem, kt % STAGES);
@@ -332,20 +333,11 @@ gemm_f64_kernel(const GemmF64Args p) {
     T.epilogue(acc);
 }
 
-// Grouped persistent form: `ngroups` independent GEMMs (one per job of a
-// batch; every group with its own sizes, operands, batch count, split-K and
-// device-side gates) share one launch.  Group g owns the tiles
-// [start[g], start[g + 1]) of a flat work list (tile t of a group is
-// (bx, by, bz) = (t % gx, (t / gx) % gy, t / (gx gy)) as in the 3-D grid of
-// gemm_f64_kernel); each CTA walks the list with stride gridDim.x and starts
-// the cp.async prologue of its next tile before it stores the current one, so
-// the loads of the next tile are in flight during the epilogue (the tiles of
-// the batch's jobs have short K ranges, where the prologue is a large share).
-// CTAs per SM the grouped kernel is compiled for (a register cap): as many as
+// CTAs per SM the persistent kernel is compiled for (a register cap): as many as
 // fit without spills: 6 (32 x 32), 3 (64 x 64 over 4 warps), 2 (64 x 64 over 8
 // warps, 128 x 64).
 template <int BM, int BN, int WARPS_M, int WARPS_N>
-constexpr int grouped_min_ctas() {
+constexpr int persistent_min_ctas() {
     return BM * BN <= 32 * 32 ? 6 : ((BM * BN <= 64 * 64 && WARPS_M * WARPS_N <= 4) ? 3 : 2);
 }
 
@@ -355,7 +347,7 @@ constexpr int grouped_min_ctas() {
 // tile routine, so it writes what gemm_f64_kernel writes; the autotuner picks
 // between the two.  The device-side gates hold for the whole launch.
 template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK, bool BKM, bool VEC>
-__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (grouped_min_ctas<BM, BN, WARPS_M, WARPS_N>()))
+__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (persistent_min_ctas<BM, BN, WARPS_M, WARPS_N>()))
 gemm_f64_persistent_kernel(const GemmF64Args p) {
     extern __shared__ __align__(16) double smem[];
     using Tile = GemmTileF64<BM, BN, BK, WARPS_M, WARPS_N, STAGES, AK, BKM, VEC>;
@@ -387,45 +379,44 @@ gemm_f64_persistent_kernel(const GemmF64Args p) {
 }
 
 
-template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK, bool BKM, bool VEC>
-__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (grouped_min_ctas<BM, BN, WARPS_M, WARPS_N>()))
+// Grouped form: `ngroups` independent GEMMs (one per job of a batch; every group
+// with its own sizes, operands, batch count, split-K and device-side gates) share
+// one launch.  Group g owns the tiles [start[g], start[g + 1]) of a flat work list
+// (tile t of a group is (bx, by, bz) = (t % gx, (t / gx) % gy, t / (gx gy)) as in the
+// 3-D grid of gemm_f64_kernel); a CTA finds its group by bisection.  One CTA per
+// tile: the tiles are short (K of 24 to 192 in a batch of water clusters), and CTAs
+// that come and go overlap one tile's epilogue with others' loads better than
+// persistent ones that start the next tile's loads themselves (T1 of (H2O)_1..8 on
+// 32 x 32 tiles 1878 against 2276 us, T2 1561 against 1869).  LOOP: fewer CTAs than
+// tiles (a context with a share of the SMs) walk the list.
+template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK, bool BKM, bool VEC, bool LOOP>
+__global__ void __launch_bounds__(32 * WARPS_M * WARPS_N)
 gemm_f64_grouped_kernel(const GemmF64Args* __restrict__ groups, const int* __restrict__ start, int ngroups) {
     extern __shared__ __align__(16) double smem[];
     using Tile = GemmTileF64<BM, BN, BK, WARPS_M, WARPS_N, STAGES, AK, BKM, VEC>;
     const int total = start[ngroups];
-    int g = 0;
-    // next tile at or after t that is not gated off; returns its index (total if none)
-    auto next = [&](int t, Tile& T) {
-        for (; t < total; t += gridDim.x) {
-            while (g + 1 < ngroups && start[g + 1] <= t) ++g;  // t only grows: advance the group
-            const GemmF64Args& p = groups[g];
-            const int lt = t - start[g];
-            const int gx = (p.M + BM - 1) / BM, gy = (p.N + BN - 1) / BN;
-            T.init(p, lt % gx, (lt / gx) % gy, lt / (gx * gy));
-            if (!T.skip) break;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        int g = 0, end = ngroups;  // start[g] <= t < start[end]
+        while (end - g > 1) {
+            const int mid = (g + end) >> 1;
+            if (start[mid] <= t) g = mid;
+            else end = mid;
         }
-        return t;
-    };
-    Tile cur;
-    int t = next(blockIdx.x, cur);
-    if (t >= total) return;
-    cur.prologue(smem);
-    typename Tile::Acc acc;
-    while (true) {
-        cur.mainloop(smem, acc);
-        Tile nxt;
-        const int tn = next(t + gridDim.x, nxt);
-        const bool more = tn < total;
-        if (more) {
-            __syncthreads();  // every warp is done with the stages the prologue overwrites
-            nxt.prologue(smem);
+        const GemmF64Args& p = groups[g];
+        const int lt = t - start[g];
+        const int gx = (p.M + BM - 1) / BM, gy = (p.N + BN - 1) / BN;
+        Tile T;
+        T.init(p, lt % gx, (lt / gx) % gy, lt / (gx * gy));
+        if (!T.skip) {
+            typename Tile::Acc acc;
+            T.prologue(smem);
+            T.mainloop(smem, acc);
+            gemm_detail::cp_async_wait<0>();
+            T.epilogue(acc);
         }
-        cur.epilogue(acc);
-        if (!more) break;
-        cur = nxt;
-        t = tn;
+        if (!LOOP) break;
+        __syncthreads();  // every warp is done with the stages the next tile overwrites
     }
-    gemm_detail::cp_async_wait<0>();
 }
 
 }  // namespace donof

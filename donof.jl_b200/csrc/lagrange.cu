@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(256, 4) build_w_fused_kernel(const double* __r
                 if (l < naux && bb < nbf5) {
                     const double* d = sd + k * nbf5;
                     double s = 0.0;
+#pragma unroll 8
                     for (int q = 0; q < nbf5; ++q) s = wbuild::tv_step(s, cj12[bb + (long long)nbf5 * q], d[q]);
                     const bool dj = (nbeta > 0) && (bb < nbeta || bb >= nalpha);
                     stv[k][tx] = wbuild::tv_value(dj, n[bb], d[bb], s);

@@ -37,3 +37,31 @@ def test_mixed_lagrangian(cuda_ctx, nbf, naux, nbeta, ncwo, nopen):
     bt.free()
     e0, h0 = native.lagrange2(C, n, H, b, cj, ck, p.nalpha, p.nbeta)
     assert rel(elag, e0) <= 2e-4 and rel(Hmat, h0) <= 1e-12
+
+
+def test_grouped_products_with_fewer_ctas_than_tiles(cuda_ctx):
+    """A context with a share of the SMs walks the grouped GEMMs' tile list: same tiles, same sums."""
+    import torch
+
+    cases = [inputs(24, 60, 5, 3, 0, 1), inputs(61, 40, 9, 4, 1, 2), inputs(96, 33, 20, 3, 0, 3)]
+    jobs = [d.eris_to_gpu(c[1], "fp64", cuda_ctx) for c in cases]
+    batch = d.Batch(jobs, [c[0] for c in cases], cuda_ctx)
+    dev = [[d.to_device(x) for x in (c[4], c[5], c[6], c[3], c[2])] for c in cases]  # n, cj, ck, H, C
+
+    def call():
+        elag = [torch.zeros(c[0].nbf, c[0].nbf, dtype=torch.float64, device="cuda") for c in cases]
+        hmat = [torch.zeros(c[0].nbf5, c[0].nbf, dtype=torch.float64, device="cuda") for c in cases]
+        batch.lagrange2(*[[x[k] for x in dev] for k in range(5)], elag, hmat)
+        torch.cuda.synchronize()
+        return [d.from_device(x) for x in elag]
+
+    whole = call()
+    cuda_ctx.set_cta_limit(7)
+    try:
+        few = call()
+    finally:
+        cuda_ctx.set_cta_limit(0)
+    batch.free()
+    for (p, b, C, H, n, cj, ck), x, y in zip(cases, whole, few):
+        assert rel(x, native.lagrange2(C, n, H, b, cj, ck, p.nalpha, p.nbeta)[0]) <= 1e-12
+        assert rel(y, x) <= 1e-14
