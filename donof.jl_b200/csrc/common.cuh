@@ -130,10 +130,9 @@ struct donof_job {
     // layout [mi + 64*n + 64*nbf*qb + 64*nbf*nb*l] with m = 64*qb + mi, nb = ceil(nbf/64)
     void* b16hi = nullptr;
     void* b16lo = nullptr;
-    // int8 digit slices of b for the FP64 form's contractions on the tensor cores
-    // (ozaki.cu): oz_b[n + ldn*(m + nbf*(l + naux*i))], followed by workspace and
-    // the row scales; oz_c holds the per-call slices and scales of C5; oz_gen counts
-    // enable/disable switches
+    // int8 digit slices of b for the FP64 form's contractions on the tensor cores,
+    // followed by the row scales (ozaki.cu); oz_c holds the per-call slices and scales
+    // of C5; oz_gen counts enable/disable switches
     void* oz_b = nullptr;
     donof::DevBuf oz_c;
     unsigned oz_gen = 0;

@@ -7,27 +7,34 @@
 //   T2   b_pq^l = C5^T tmp_l
 //   Y    Y      = sum_l tmp_l W_l  (the restructured Lagrangian of lagrange.cu)
 //
-// Digits.  A number x with |x| <= F s (F = 0.498) is written as S signed 8-bit
-// digits, x = s sum_{i<S} d_i 256^-(i+1), d_i in [-128, 127]: with the integer
-// X = rint(x / s 2^(8S)) the bytes of X + sum_i 128 256^i are d_i + 128, so one
-// 64-bit addition yields every digit.  The residual is rounded to nearest
-// (no sign correlation between the dropped parts of the two operands), and the
-// scales are the largest |x| itself, not a power of two above it.
-//   b     6 digits, one scale per row m of b_l               (made once per job)
-//   C5    6 digits, one scale per column q                   (per call)
-//   tmp   7 digits, scale RL[l] CN[q]: the largest row norm of b_l times the norm
+// Digits.  T1's operands are seven signed 7-bit digits below a power of two,
+//     x = 2^e sum_{i<7} d_i 2^(-7(i+1)),   d_i = trunc(128 r_i), r_(i+1) = 128 r_i - d_i,
+// with 2^e the smallest power of two above the row's (column's) largest |x|.  The
+// others are seven balanced 8-bit digits below any scale s, |x| <= F s (F = 0.498),
+//     x = s sum_{i<7} d_i 256^-(i+1),   d_i in [-128, 127]:
+// with the integer X = rint(x / s 2^56) the bytes of X + sum_i 128 256^i are d_i + 128,
+// so one 64-bit addition yields every digit, and the residual is rounded to nearest.
+//   b, C5 (T1)  truncated digits, one scale per row m of b_l (made once per job) and
+//         per column q
+//   C5 (T2)     balanced digits, one scale per column
+//   tmp   balanced, scale RL[l] CN[q]: the largest row norm of b_l times the norm
 //         of column q bounds |tmp_l[m, q]| (Cauchy-Schwarz), so the digits are
 //         written by T1's epilogue with no pass for a maximum; the bound is 2-3
-//         bits above the largest value, which the seventh digit pays for
-//   W     7 digits of RL[l] CN[q] W_l[q, b], one scale per b (beta_b times the
+//         bits above the largest value
+//   W     balanced digits of RL[l] CN[q] W_l[q, b], one scale per b (beta_b times the
 //         largest |RL CN b_pq| and |RL CN t|, found by T2's epilogue and the
 //         diagonal kernel), so that tmp's scales drop out of Y's sum over (q, l)
-// A product keeps the digit pairs with i + j < G = 7: exact s8 x s8 -> s32 sums
-// (tcgen05.mma kind::i8) in 7 TMEM accumulators (one per i + j, 64 columns each),
-// combined in FP64 by the epilogue (exact int32 -> double, Horner in 2^-8).
-// |sum| <= 7 * 2^14 * K < 2^31 for K <= 18688; Y's K range is cut accordingly.
+// A product keeps the digit pairs with i + j < NG, NG = 7 in T1 and 8 in T2 and Y:
+// exact s8 x s8 -> s32 sums (tcgen05.mma kind::i8) in NG TMEM accumulators (one per
+// i + j, 64 columns each), combined in FP64 by the epilogue (exact int32 -> double,
+// Horner in 2^-7 or 2^-8).  |sum| <= 7 * 2^14 * K < 2^31 for K <= 18688; Y's K range is
+// cut accordingly.
+// T1 is within 1e-13 of the FP64 product, T2 and Y are as near to theirs as an FP64
+// GEMM (error of b_pq 1.4e-16 of the norm, of Y 2.1e-16, the GEMM's 3.3e-16 and
+// 9.7e-16, nbf = 96, random b; NG = 7 left 1.6e-15 in Y).  The optimisers divide by
+// gradient elements, so noise of 1e-14 in T2 and Y showed as 1e-8 in the orbitals.
 //
-// One persistent kernel, oz_kernel<MODE>, with TMEM accumulators 7 x 64 columns
+// One persistent kernel, oz_kernel<MODE>, with TMEM accumulators of 64 columns each
 // for a 128 x 64 output tile: warp 16 streams A's slices (16 KB TMA boxes, no
 // multicast) through a ring, warp 17 issues the MMAs, warps 0-15 drain TMEM.
 // B's slices are adjacent in shared memory, so the products of one A slice with
@@ -38,18 +45,20 @@
 //   Y:  rows m, K = (q, l).  A = the same slices of tmp read K-major, B = W's;
 //       a unit is (tile, K range), its FP64 partial left for the tail to sum.
 // T1 and T2 keep the C5 slices of the CTA's column tile in shared memory for the
-// whole launch where they fit (nbf <= 384); a CTA then serves one column tile.
+// whole launch where they fit (nbf <= 256); a CTA then serves one column tile.
 //
-// Measured on one B200 (us; in brackets T1 from 7-bit digits, T2 and Y as FP64 GEMMs):
+// Measured on one B200 (us; in brackets T1 alone from digits, T2 and Y as FP64 GEMMs):
 //   nbf / naux / nbf5    T1            T2            W            Y            Lagrangian
-//   256 / 1024 / 64      104 (131)     40 (85)       21 (20)      32 (81)      (orbital step 289 (393))
-//   202 / 974 / 198      264 (470)     308 (761)     149 (186)    231 (841)    1029 (2231)
-//   384 / 1856 / 320     1700 (2049)   1541 (4649)   600 (698)    1266 (6958)  5848 (14295)
-// At nbf5 = 64 T1 is bound by HBM (b's slices in, tmp's out: 520 MB, 81 us at 6.45
+//   256 / 1024 / 64      110 (131)     40 (85)       23 (20)      31 (81)      (orbital step 345 (433))
+//   202 / 974 / 198      268 (470)     318 (761)     144 (186)    234 (841)    1139 (2238)
+//   384 / 1856 / 320     1774 (2049)   1697 (4649)   553 (698)    1399 (6958)  6496 (14355)
+// (the kernels one by one; the Lagrangian in a loop, at the 1.74 GHz of the power cap).
+// At nbf5 = 64 T1 is bound by HBM (b's slices in, tmp's out: 587 MB, 91 us at 6.45
 // TB/s); the larger ones by what the MMAs and the TMA need of shared memory (a
-// chunk of Y: 384 KB of operand reads, 168 KB written, 4300 cycles at 128 bytes a
-// cycle; 5100 measured) and, in T1 and T2, by the drain between two rounds.
-// The error against 64 bits fell from 7.2e-14 to 6.3e-15 of the norm of elag.
+// chunk of Y: 448 KB of operand reads, 168 KB written, 4900 cycles at 128 bytes a
+// cycle; 5200 measured) and, in T1 and T2, by the drain between two rounds.
+// elag is within 1e-15 of what the FP64 GEMMs make of the same tmp; its error against
+// 64 bits, 7.2e-14 of the norm, is that of T1's truncated digits.
 //
 // Every wait is bounded; on a timeout the CTA records the failure in the
 // context's failure word, drains its copies and MMAs, frees TMEM and exits.
@@ -67,10 +76,9 @@ namespace donof {
 
 namespace oz {
 
-constexpr int SB = 6;                       // digits of b and of C5
-constexpr int SW = 7;                       // digits of tmp and of W
-constexpr int NG = 7;                       // accumulators: digit pairs with i + j < NG
-constexpr double F = 0.498;                 // largest |x| / scale: every digit fits [-128, 127]
+constexpr int S = 7;                        // digits of every operand
+constexpr int NG_MAX = 8;                   // accumulators: digit pairs with i + j < NG
+constexpr double F = 0.498;                 // largest |x| / scale: every balanced digit fits [-128, 127]
 constexpr int EPI_WARPS = 16;               // four per TMEM lane quarter, 16 columns each (8 of 32: T1 148 against 113 us at nbf5 = 64)
 constexpr int PRODUCER = EPI_WARPS;         // TMA producer
 constexpr int ISSUER = EPI_WARPS + 1;       // TMEM allocator + MMA issuer
@@ -89,7 +97,7 @@ constexpr int OFF_DATA = 1024;              // B stages, then the A ring
 constexpr int DATA_BYTES = 224 * 1024;
 constexpr int SMEM_ALLOC = OFF_DATA + DATA_BYTES + 1024;  // slack for 1024-B alignment
 static_assert(SMEM_ALLOC <= 227 * 1024, "shared memory budget");
-static_assert(NG * QT <= 512, "TMEM columns");
+static_assert(NG_MAX * QT <= 512, "TMEM columns");
 constexpr int KMAX_CHUNKS = 146;            // 7 * 2^14 * 146 * 128 < 2^31
 static_assert(7ll * 16384 * KMAX_CHUNKS * KC < (1ll << 31), "int32 accumulators");
 
@@ -99,9 +107,9 @@ constexpr int A_EMPTY = RING_MAX;           // +s: A stage consumed by the MMAs
 constexpr int B_FULL = 2 * RING_MAX;        // +stage: B stage landed (resident: one per K chunk)
 constexpr int B_STAGES = 8;
 constexpr int B_EMPTY = B_FULL + B_STAGES;  // +slot (2): streamed B stage consumed
-constexpr int ACC_FULL = B_EMPTY + 2;       // accumulators of a round complete: +0 the last (6), +1 5..3, +2 2..0
-constexpr int GFREE = ACC_FULL + 3;         // +g (NG): accumulator g drained and zeroed (count EPI_WARPS)
-constexpr int B_END = GFREE + NG;           // every MMA of the CTA complete
+constexpr int ACC_FULL = B_EMPTY + 2;       // accumulators of a round complete: +0 the last, +1 those from 4 on, +2 3..0
+constexpr int GFREE = ACC_FULL + 3;         // +g (NG_MAX): accumulator g drained and zeroed (count EPI_WARPS)
+constexpr int B_END = GFREE + NG_MAX;       // every MMA of the CTA complete
 static_assert((B_END + 1) * 8 <= OFF_MISC, "barrier area");
 
 enum Mode {
@@ -110,6 +118,8 @@ enum Mode {
     T2 = 2,         // b_pq in FP64
     YSUM = 3,       // FP64 partials of Y
 };
+
+constexpr int accumulators(int mode) { return mode == T2 || mode == YSUM ? 8 : 7; }
 
 struct Params {
     int nbf, nbf5, naux, ldq;  // ldq: nbf5 rounded up to 16 (row length of tmp's and W's slices per l)
@@ -120,11 +130,13 @@ struct Params {
     int resident;              // B's stages of the CTA's column tile are loaded once and kept
     int ring;                  // A stages
     int ring_off;              // byte offset of the ring behind OFF_DATA
-    const double* ra;          // sa / RL per row (m, l) of b
+    const double* sa;          // 2^ea per row (m, l) of b
     const double* RL;          // per l
+    const double* RLi;         // per l: 1 / RL (0 for b_l = 0)
     const double* CN;          // per q
-    const double* cb;          // per q: sb 2^40 / CN
-    const double* sb2;         // per q: sb 2^-16
+    const double* cb;          // per q: 2^(eb - 14) 2^56 / CN
+    const double* sb1;         // per q: 2^(eb - 14), of C5's truncated digits
+    const double* sb2;         // per q: s 2^-16, of its balanced digits
     const double* beta;        // per b (Y)
     unsigned* wmax;            // [0] of |RL CN b_pq|, [1] of |RL CN t| / beta: high words of the largest value
     int8_t* t8;                // tmp's slices (see the layout above t8_at)
@@ -146,10 +158,10 @@ __device__ __forceinline__ double exact_f64(int x) {
 // Layout of the slices (the MMAs read them without swizzle): 128-wide chunks of the
 // contiguous index (R = q + ldq l of tmp and W, n of b and C5), each in eight groups
 // of 16, a group's 16 bytes contiguous and the rows one 16-byte step apart.
-//   b    b8[n % 16 + 16 (r % 128 + 128 (n / 16 + ldn/16 (i + 6 (r / 128))))]   r = m + nbf l
+//   b    b8[n % 16 + 16 (r % 128 + 128 (n / 16 + ldn/16 (i + 7 (r / 128))))]   r = m + nbf l
 //   tmp  t8[R % 16 + 16 (m + nbf (g + 8 (i + 7 chunk)))]      g = R / 16 % 8, chunk = R / 128
 //   W    w8[R % 16 + 16 (b + nbf5 (j + 7 (g + 8 chunk)))]
-//   C5   c8[n % 16 + 16 (q + nbf5 (j + 6 (g + 8 chunk)))]
+//   C5   c8[n % 16 + 16 (q + nbf5 (j + 7 (g + 8 chunk)))]  (two: truncated and balanced)
 // A row step of 16 bytes makes the stores contiguous over a warp's rows (512 bytes an
 // instruction: with rows 128 bytes apart W's kernel took 185 instead of 126 us at
 // nbf5 = 198), gives the 8 x 16-byte core matrices that a K-major and an MN-major
@@ -157,7 +169,7 @@ __device__ __forceinline__ double exact_f64(int x) {
 // group.  A box is rows of 2 KB: T1's loads alone took 234 us at nbf = 202 as 128
 // swizzled rows of 128 bytes at a pitch of 208, and take 160 us so.
 __device__ __forceinline__ size_t t8_at(int R, int m, int nbf) {  // digit 0; digit i: + 128 nbf i
-    return 16 * ((size_t)nbf * ((size_t)(R >> 7) * 8 * SW + ((R >> 4) & 7)) + m) + (R & 15);
+    return 16 * ((size_t)nbf * ((size_t)(R >> 7) * 8 * S + ((R >> 4) & 7)) + m) + (R & 15);
 }
 
 // The seven digits of z (|z| <= F 2^56) as bytes: byte 6 - i is digit i.
@@ -167,7 +179,7 @@ __device__ __forceinline__ unsigned long long digits7(double z) {
 }
 
 // Byte transposition of four 7-byte digit strings: w[i] = digit i of z0, z1, z2, z3.
-__device__ __forceinline__ void pack4(const unsigned long long (&z)[4], unsigned (&w)[SW]) {
+__device__ __forceinline__ void pack4(const unsigned long long (&z)[4], unsigned (&w)[S]) {
     const unsigned a0 = (unsigned)z[0], a1 = (unsigned)z[1], a2 = (unsigned)z[2], a3 = (unsigned)z[3];
     const unsigned h0 = (unsigned)(z[0] >> 32), h1 = (unsigned)(z[1] >> 32), h2 = (unsigned)(z[2] >> 32),
                    h3 = (unsigned)(z[3] >> 32);
@@ -264,14 +276,15 @@ __device__ __forceinline__ Unit unit_of(const Params& P, int u) {
 // behind them arrives on.  i and part are constants after unrolling; the branch on
 // nk4 stays outside the elected lane's region, which is straight code (an MMA takes
 // about 80 issue cycles, 92 to execute: what the warp does between them counts).
-template <int MODE, int NB>
+template <int MODE>
 __device__ __forceinline__ void issue_slice(int i, int part, uint32_t tmem, uint64_t ad, uint64_t bd, int nk4,
                                             uint32_t done) {
-    const int cnt = (NG - i) < NB ? (NG - i) : NB;
+    constexpr int NG = accumulators(MODE);
+    const int cnt = (NG - i) < S ? (NG - i) : S;
     const int first = cnt <= 4 ? cnt : (cnt + 1) / 2;
     // 32 K further: two groups, or for the MN-major operand four 8-row core matrices
     constexpr uint64_t astep = (MODE == T2 ? 32 * 16 : 2 * 16 * MT) >> 4;
-    constexpr uint64_t bstep = (2 * 16 * NB * QT) >> 4;
+    constexpr uint64_t bstep = (2 * 16 * S * QT) >> 4;
     constexpr uint32_t amn = MODE == T2 ? 1u << 15 : 0u;
     auto step = [&](int k4) {
         if (part & 1)
@@ -310,31 +323,29 @@ __device__ __forceinline__ uint64_t a_desc(uint32_t addr) {
     if (MODE == T2) return sdesc_flat(addr, 128, 16 * MT);  // MN-major: (q, l) along M, 8 m per 128 bytes
     return sdesc_flat(addr, 16 * MT, 128);                  // K-major: groups of 16 K 2 KB apart
 }
-template <int NB>
 __device__ __forceinline__ uint64_t b_desc(uint32_t addr) {
-    return sdesc_flat(addr, 16 * NB * QT, 128);
+    return sdesc_flat(addr, 16 * S * QT, 128);
 }
 
-// Round r of a CTA = one unit: its MMAs accumulate into the 7 accumulators, then
+// Round r of a CTA = one unit: its MMAs accumulate into the NG accumulators, then
 // the epilogue drains them.  A's slices are consumed from the least significant
-// (i = NA - 1) to the most: slice i writes accumulators i .. 6 only, so the first
+// (i = 6) to the most: slice i writes accumulators i .. i + 6 only, so the first
 // MMAs of round r + 1 need only the top accumulators, which the epilogue of round
 // r drains (and zeroes) first.  The drain of accumulator g is a TMEM load and a
 // store of zeros; its release (GFREE[g]) comes right after, and the FP64
 // arithmetic of the epilogue runs while the next round's MMAs already fill the
 // released columns.
-// With B resident (NKC = its K chunks, 1 to 3) the order is slice-major over the K
-// chunks, and a round ends with slice 0 against B's upper slices (accumulators 5..3),
-// then its lower ones (2..0): accumulator 6 is complete a slice earlier, 5..3 half a
-// slice earlier, so the epilogue drains them while the last MMAs run and the tensor
+// With B resident (NKC = its K chunks, 1 or 2) the order is slice-major over the K
+// chunks, and a round ends with slice 0 against B's upper slices (accumulators 6..4),
+// then its lower ones (3..0): accumulator 7 (NG = 8) is complete a slice earlier, 6..4
+// half a slice earlier, so the epilogue drains them while the last MMAs run and the tensor
 // cores do not wait for it between rounds.  With B streamed (NKC = 0) the order is
 // chunk by chunk.
 template <int MODE, int NKC>
 __global__ void __launch_bounds__(BOUND_THREADS, 1)
 oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params P) {
-    constexpr int NA = (MODE == T2 || MODE == YSUM) ? SW : SB;
-    constexpr int NB = (MODE == YSUM) ? SW : SB;
-    constexpr int B_BYTES = NB * BS_BYTES;
+    constexpr int NG = accumulators(MODE);
+    constexpr int B_BYTES = S * BS_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t sbase = saddr(sm) + OFF_DATA;
@@ -353,11 +364,10 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     constexpr bool resident = NKC > 0;
     const int my_units = unit_count<MODE, resident>(P);
-    static_assert(!(resident && NB == NG), "accumulator 6 must be complete before slice 0");
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        for (int i = 0; i <= B_END; ++i) mbar_init(bar(i), (i >= GFREE && i < GFREE + NG) ? EPI_WARPS : 1);
+        for (int i = 0; i <= B_END; ++i) mbar_init(bar(i), (i >= GFREE && i < GFREE + NG_MAX) ? EPI_WARPS : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == ISSUER) {
@@ -382,11 +392,11 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                 if (elect_one()) {
                     mbar_expect_tx(bar(A_FULL + s), (uint32_t)A_BYTES);
                     if (MODE == T2)  // 128 m (K) of the 128 (q, l) of a row tile
-                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * kc * KC, 0, i + SW * row);
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * kc * KC, 0, i + S * row);
                     else if (MODE == YSUM)  // 128 (q, l) (K) of 128 m
-                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * row * MT, 0, i + SW * kc);
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 2 * row * MT, 0, i + S * kc);
                     else  // 128 n (K) of 128 (m, l)
-                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 0, 8 * kc, i + SB * row);
+                        tma_load_3d(sring + s * A_BYTES, &map_a, bar(A_FULL + s), 0, 8 * kc, i + S * row);
                 }
                 __syncwarp();
                 ++it;
@@ -410,7 +420,7 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
             for (int u = 0; u < my_units && ok; ++u) {
                 const Unit w = unit_of<MODE, resident>(P, u);
                 if (resident) {
-                    for (int i = NA - 1; i >= 0 && ok; --i)
+                    for (int i = S - 1; i >= 0 && ok; --i)
                         for (int kc = 0; kc < w.nc && ok; ++kc) ok = load_a(i, kc, w.row);
                     continue;
                 }
@@ -421,7 +431,7 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                         break;
                     }
                     load_b(slot, w.col, kc);
-                    for (int i = NA - 1; i >= 0 && ok; --i) ok = load_a(i, kc, w.row);
+                    for (int i = S - 1; i >= 0 && ok; --i) ok = load_a(i, kc, w.row);
                 }
             }
             // drain: every issued copy has landed before the CTA exits
@@ -473,8 +483,8 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
 #pragma unroll
                         for (int kc = 0; kc < NKC; ++kc) ok = ok && wait(B_FULL + kc, 0);
 #pragma unroll
-                    for (int ii = 0; ii < NA; ++ii) {
-                        const int i = NA - 1 - ii;
+                    for (int ii = 0; ii < S; ++ii) {
+                        const int i = S - 1 - ii;
                         if (ii == 0)
                             for (int g = NG - 1; g >= i; --g) ok = ok && wait(GFREE + g, up);
                         else if (!__all_sync(0xffffffffu, gready))
@@ -490,26 +500,27 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                             next();
                             if (i > 0 && kc == NKC - 1) gready = mbar_test(bar(GFREE + i - 1), up);
                             fence_after();
-                            const uint64_t bd = b_desc<NB>(sbase + kc * B_BYTES);
+                            const uint64_t bd = b_desc(sbase + kc * B_BYTES);
                             const int nk4 = kc == NKC - 1 ? P.k4_last : KC / 32;
                             if (i > 0) {
-                                issue_slice<MODE, NB>(i, 3, tmem, d, bd, nk4, done);
+                                issue_slice<MODE>(i, 3, tmem, d, bd, nk4, done);
                             } else {
-                                issue_slice<MODE, NB>(0, 2, tmem, d, bd, nk4, 0);
+                                issue_slice<MODE>(0, 2, tmem, d, bd, nk4, 0);
                                 db[kc] = done;
                                 da[kc] = d;
                             }
                         }
                         if (!ok) break;
-                        if (i == 1) {
+                        if (i == NG - S) {  // slice 1 (NG = 8) or the upper part of slice 0: the last accumulator
                             if (elect_one()) umma_commit(bar(ACC_FULL));
                             __syncwarp();
-                        } else if (i == 0) {
+                        }
+                        if (i == 0) {
                             if (elect_one()) umma_commit(bar(ACC_FULL + 1));
                             __syncwarp();
 #pragma unroll
                             for (int kc = 0; kc < NKC; ++kc)
-                                issue_slice<MODE, NB>(0, 1, tmem, da[kc], b_desc<NB>(sbase + kc * B_BYTES),
+                                issue_slice<MODE>(0, 1, tmem, da[kc], b_desc(sbase + kc * B_BYTES),
                                                       kc == NKC - 1 ? P.k4_last : KC / 32, db[kc]);
                             if (elect_one()) umma_commit(bar(ACC_FULL + 2));
                             __syncwarp();
@@ -520,18 +531,18 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                     for (int g = NG - 1; g >= 0; --g) ok = ok && wait(GFREE + g, up);
                     for (int kc = w.c0; kc < w.c0 + w.nc && ok; ++kc, ++bs) {
                         const int slot = bs & 1;
-                        const uint64_t bd = b_desc<NB>(sbase + slot * B_BYTES);
+                        const uint64_t bd = b_desc(sbase + slot * B_BYTES);
                         const int nk4 = kc == P.nkc - 1 ? P.k4_last : KC / 32;
                         ok = wait(B_FULL + slot, (uint32_t)((bs >> 1) & 1));
 #pragma unroll
-                        for (int ii = 0; ii < NA; ++ii) {
+                        for (int ii = 0; ii < S; ++ii) {
                             ok = ok && landed();
                             if (!ok) break;
                             const uint32_t done = fb + 8u * RING_MAX;
                             const uint64_t d = ad;
                             next();
                             fence_after();
-                            issue_slice<MODE, NB>(NA - 1 - ii, 3, tmem, d, bd, nk4, done);
+                            issue_slice<MODE>(S - 1 - ii, 3, tmem, d, bd, nk4, done);
                         }
                         if (ok && elect_one()) umma_commit(bar(B_EMPTY + slot));
                         __syncwarp();
@@ -584,15 +595,16 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                 l = R / P.nbf;
                 x = R - l * P.nbf;
                 in = l < P.naux;
-                if (in) rs = MODE == T1_F64 ? P.ra[R] * P.RL[l] : P.ra[R];
+                if (in) rs = MODE == T1_F64 ? P.sa[R] : P.sa[R] * P.RLi[l];
             }
-            // Horner in 2^-8 from the least significant accumulator: v = sum_g acc_g 2^(-8g)
+            // Horner from the least significant accumulator: v = sum_g acc_g 2^(-8g), or 2^(-7g)
+            constexpr double radix = MODE == T2 || MODE == YSUM ? 0x1p-8 : 0x1p-7;
             double v[NC];
             bool ok = true;
 #pragma unroll
             for (int g = NG - 1; g >= 0; --g) {
-                if (g == 6 || g == 5 || g == 2) {
-                    ok = ok && wait(ACC_FULL + (g == 6 ? 0 : g == 5 ? 1 : 2), (uint32_t)(u & 1));
+                if (g == NG - 1 || g == NG - 2 || g == 3) {
+                    ok = ok && wait(ACC_FULL + (g == NG - 1 ? 0 : g == NG - 2 ? 1 : 2), (uint32_t)(u & 1));
                     if (!ok) break;
                     fence_after();
                 }
@@ -607,14 +619,14 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
 #pragma unroll
                 for (int k = 0; k < NC; ++k) {
                     const double t = exact_f64((int)a[k]);
-                    v[k] = (g == NG - 1) ? t : fma(v[k], 0x1p-8, t);
+                    v[k] = (g == NG - 1) ? t : fma(v[k], radix, t);
                 }
             }
             if (!ok) break;
             if (MODE == T1_DIGITS) {
                 // digit slices of tmp, q contiguous: 16 bytes per slice and thread; the
                 // padding columns [nbf5, ldq) get cb = 0, i.e. zero digits
-                unsigned wd[4][SW];
+                unsigned wd[4][S];
 #pragma unroll
                 for (int k4 = 0; k4 < 4; ++k4) {
                     unsigned long long z[4];
@@ -625,7 +637,7 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                 if (in && q0 < P.ldq) {
                     int8_t* dst = P.t8 + t8_at(P.ldq * l + q0, x, P.nbf);
 #pragma unroll
-                    for (int i = 0; i < SW; ++i)
+                    for (int i = 0; i < S; ++i)
                         *reinterpret_cast<uint4*>(dst + (size_t)i * P.nbf * 128) =
                             make_uint4(wd[0][i], wd[1][i], wd[2][i], wd[3][i]);
                 }
@@ -633,7 +645,7 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                 double* dst = P.out + (size_t)P.nbf * P.nbf5 * l + x;
 #pragma unroll
                 for (int k = 0; k < NC; ++k)
-                    if (in && q0 + k < P.nbf5) dst[(size_t)P.nbf * (q0 + k)] = v[k] * rs * P.sb2[q0 + k];
+                    if (in && q0 + k < P.nbf5) dst[(size_t)P.nbf * (q0 + k)] = v[k] * rs * P.sb1[q0 + k];
             } else if (MODE == T2) {
 #pragma unroll
                 for (int k = 0; k < NC; ++k) {
@@ -682,20 +694,30 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------- digit slices
-// The six digits of x / s (|x| <= F s) as bytes: byte 5 - i is digit i.
-__device__ __forceinline__ unsigned long long digits6(double x, double s) {
-    const unsigned long long bias = 0x0000808080808080ull;
-    return (unsigned long long)(__double2ll_rn(x / s * 0x1p48) + (long long)bias) ^ bias;
+// The seven balanced digits of x / s (|x| <= F s) as bytes: byte 6 - i is digit i.
+__device__ __forceinline__ unsigned long long digits7(double x, double s) { return digits7(x / s * 0x1p56); }
+
+// The seven truncated digits of y, |y| < 1: d_i = trunc(128 r_i), r_(i+1) = 128 r_i - d_i.
+__device__ __forceinline__ unsigned long long truncated7(double y) {
+    unsigned long long z = 0;
+#pragma unroll
+    for (int i = 0; i < S; ++i) {
+        y *= 128.0;
+        const double t = trunc(y);
+        z = z << 8 | (unsigned)((int)t & 255);
+        y -= t;
+    }
+    return z;
 }
 
-// The digit scale of a row or column whose largest |x| is mx (floored, so that
-// x / s never overflows; a zero row has zero digits whatever its scale).
+// The scale of balanced digits of a column whose largest |x| is mx (floored, so that
+// x / s never overflows; a zero column has zero digits whatever its scale).
 __device__ __forceinline__ double digit_scale(double mx) { return fmax(mx, 1e-280) / F; }
 
-// Per row (m, l) of b: sa = digit_scale(max_n |b|) into ra (made sa / RL by
-// row_finish_kernel) and the row norm's maximum over m into rn[l] (bits of a
-// non-negative double).  One thread per (m, l), coalesced over m.
-__global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long long naux, double* __restrict__ ra,
+// Per row (m, l) of b: sa = 2^e with max_n |b| < 2^e (1 for a zero row), and the row
+// norm's maximum over m into rn[l] (bits of a non-negative double).  One thread per
+// (m, l), coalesced over m.
+__global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long long naux, double* __restrict__ sa,
                                  unsigned long long* __restrict__ rn) {
     const long long total = (long long)nbf * naux;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -718,27 +740,27 @@ __global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long lon
             }
             norm = mx * sqrt(ss);
         }
-        ra[i] = digit_scale(mx);
+        int e = 0;
+        if (mx > 0.0) frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1)
+        sa[i] = isnan(norm) || isinf(mx) ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, e);
         atomicMax(rn + l, (unsigned long long)__double_as_longlong(norm));
     }
 }
 
-// rn[l] (bits) -> RL[l] = norm (1 + 2^-30) / F in place, ra = sa / RL (0 for b_l = 0)
-__global__ void row_finish_kernel(int nbf, long long naux, const unsigned long long* __restrict__ rn,
-                                  double* __restrict__ RL, double* __restrict__ ra) {
-    const long long total = (long long)nbf * naux;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long l = i / nbf;
-        const double R = __longlong_as_double((long long)rn[l]) * (1.0 + 0x1p-30) / F;
-        if (i == l * nbf) RL[l] = R;
-        ra[i] = R > 0.0 ? ra[i] / R : 0.0;
+// rn[l] (bits) -> RL[l] = norm (1 + 2^-30) / F, RLi = 1 / RL in rn's place
+__global__ void row_finish_kernel(long long naux, double* __restrict__ RL, double* __restrict__ rn) {
+    for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < naux;
+         l += (long long)gridDim.x * blockDim.x) {
+        double R = rn[l] * (1.0 + 0x1p-30) / F;
+        if (R > 0.0 && R < 1e-290) R = 1e-290;  // 1 / R stays finite
+        RL[l] = R;                              // NaN where b_l holds one: b_pq and Y follow
+        rn[l] = R > 0.0 ? 1.0 / R : 0.0;
     }
 }
 
 // b's slices (layout above t8_at), n < ldn = nbf rounded up to 16.  32 x 32 (m, n)
 // tiles through shared memory: reads coalesced over m, four n of one digit a 4-byte
-// word.  s = digit_scale of the row.
+// word.
 __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__ b, const double* __restrict__ sa,
                                                       int nbf, int ldn, long long naux, int8_t* __restrict__ out) {
     __shared__ double tile[32][33];
@@ -763,13 +785,13 @@ __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__
             const double s = sa[m + (long long)nbf * l];
             unsigned long long z[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) z[k] = digits6(tile[nq + k][m - m0], s) << 8;
-            unsigned w[SW];
-            pack4(z, w);  // digit i of the 6 is byte 6 - i of the shifted string
+            for (int k = 0; k < 4; ++k) z[k] = truncated7(tile[nq + k][m - m0] / s);
+            unsigned w[S];
+            pack4(z, w);
             const long long row = m + (long long)nbf * l;
-            int8_t* dst = out + 16 * ((row & 127) + 128 * (((n0 + nq) >> 4) + (long long)(ldn / 16) * SB * (row >> 7))) + (nq & 15);
+            int8_t* dst = out + 16 * ((row & 127) + 128 * (((n0 + nq) >> 4) + (long long)(ldn / 16) * S * (row >> 7))) + (nq & 15);
 #pragma unroll
-            for (int i = 0; i < SB; ++i) *reinterpret_cast<unsigned*>(dst + 128ll * ldn * i) = w[i];
+            for (int i = 0; i < S; ++i) *reinterpret_cast<unsigned*>(dst + 128ll * ldn * i) = w[i];
         }
     }
 }
@@ -778,12 +800,12 @@ struct PrepArgs {
     const double* C;
     const double *n, *cj12, *ck12;  // null: no W will be built
     int nbf, nbf5, nkc;             // grid: the columns rounded up to whole tiles
-    double *sb2, *CN, *cb, *beta;
-    int8_t* out;                    // c8, n padded to whole chunks with zeros
+    double *sb1, *sb2, *CN, *cb, *beta;
+    int8_t *c1, *c2;                // c8 of T1 and of T2, n padded to whole chunks with zeros
     unsigned* wmax;
 };
 
-// One block per column q of C5 (and per padding column): its digit slices, the
+// One block per column q of C5 (and per padding column): both sets of digit slices, the
 // scales of T1 and T2, and beta_q = the largest |factor| of W's column q.
 __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
     __shared__ double red[3][4];
@@ -791,7 +813,7 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
     const int q = blockIdx.x, tid = threadIdx.x;
     if (q == 0 && tid < 2) a.wmax[tid] = 0;
     if (q >= a.nbf5) {
-        if (tid == 0) a.sb2[q] = a.CN[q] = a.cb[q] = a.beta[q] = 0.0;
+        if (tid == 0) a.sb1[q] = a.sb2[q] = a.CN[q] = a.cb[q] = a.beta[q] = 0.0;
         return;
     }
     const double* col = a.C + (long long)a.nbf * q;
@@ -827,6 +849,9 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
     be = reduce(be, 1, false);
     const bool anybad = __syncthreads_or(bad);
     const double s = digit_scale(mx);
+    int e = 0;
+    if (mx > 0.0) frexp(mx, &e);
+    const double inv = ldexp(1.0, -e);
     double ss = 0.0;
     for (int n = tid; n < a.nbf; n += blockDim.x) {
         const double x = col[n] / s;
@@ -838,15 +863,20 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
         double cn = s * sqrt(ss) * (1.0 + 0x1p-40);
         if (!isfinite(ss) || isinf(mx)) cn = nan;  // a column with a NaN or an infinity: every product of it is NaN
         a.CN[q] = cn;
+        a.sb1[q] = isnan(cn) ? nan : ldexp(1.0, e - 14);  // 2^-14: the weight of digit pair (0, 0)
         a.sb2[q] = isnan(cn) ? nan : s * 0x1p-16;
-        a.cb[q] = cn == 0.0 ? 0.0 : s * 0x1p40 / cn;
+        a.cb[q] = cn == 0.0 ? 0.0 : ldexp(1.0, e - 14) * 0x1p56 / cn;
         a.beta[q] = anybad ? nan : be;
     }
     for (int n = tid; n < a.nkc * KC; n += blockDim.x) {
-        const unsigned long long z = n < a.nbf ? digits6(col[n], s) : 0ull;
-        int8_t* dst = a.out + (n & 15) + 16 * (q + (long long)a.nbf5 * SB * (n >> 4));
+        const double x = n < a.nbf ? col[n] : 0.0;
+        const unsigned long long z1 = truncated7(x * inv), z2 = digits7(x, s);
+        const long long at = (n & 15) + 16 * (q + (long long)a.nbf5 * S * (n >> 4));
 #pragma unroll
-        for (int i = 0; i < SB; ++i) dst[16ll * a.nbf5 * i] = (int8_t)(z >> (8 * (SB - 1 - i)));
+        for (int i = 0; i < S; ++i) {
+            a.c1[at + 16ll * a.nbf5 * i] = (int8_t)(z1 >> (8 * (S - 1 - i)));
+            a.c2[at + 16ll * a.nbf5 * i] = (int8_t)(z2 >> (8 * (S - 1 - i)));
+        }
     }
 }
 
@@ -931,7 +961,7 @@ __global__ void __launch_bounds__(256) w_digits_kernel(const double* __restrict_
         const double sc = w_scale(beta[b], wmax);
         const double f = (sc == 0.0 || !in) ? 0.0 : RL[l] * (F * 0x1p56 / sc);
         const double td = (in && b >= q0 && b < q0 + 16) ? tv[b + (long long)nbf5 * l] : 0.0;
-        unsigned wd[4][SW];
+        unsigned wd[4][S];
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
             unsigned long long z[4];
@@ -948,9 +978,9 @@ __global__ void __launch_bounds__(256) w_digits_kernel(const double* __restrict_
             }
             pack4(z, wd[k4]);
         }
-        int8_t* dst = W8 + 16 * ((long long)nbf5 * SW * t + b);
+        int8_t* dst = W8 + 16 * ((long long)nbf5 * S * t + b);
 #pragma unroll
-        for (int j = 0; j < SW; ++j)
+        for (int j = 0; j < S; ++j)
             *reinterpret_cast<uint4*>(dst + 16ll * nbf5 * j) = make_uint4(wd[0][j], wd[1][j], wd[2][j], wd[3][j]);
     }
 }
@@ -961,32 +991,32 @@ namespace {
 
 int ldn_of(int nbf) { return (nbf + 15) / 16 * 16; }  // 16-byte row pitch (TMA stride rule)
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-// one slice of b (whole 128-row tiles); the job's buffer holds the SB slices, one
-// slice's worth of workspace (W's digit slices, where they fit), ra and RL
+// one slice of b (whole 128-row tiles); the job's buffer holds the S slices, sa, RL and RLi
 size_t slice_bytes(int nbf, int naux) { return ((size_t)naux * nbf + oz::MT - 1) / oz::MT * oz::MT * ldn_of(nbf); }
 
 struct JobLayout {
-    size_t work, ra, rl, bytes;
+    size_t sa, rl, bytes;
 };
 JobLayout job_layout(int nbf, int naux) {
     JobLayout o;
-    o.work = align256(oz::SB * slice_bytes(nbf, naux));
-    o.ra = o.work + align256(slice_bytes(nbf, naux));
-    o.rl = o.ra + align256(sizeof(double) * (size_t)nbf * naux);
-    o.bytes = o.rl + sizeof(double) * 2 * (size_t)naux;  // RL, and the bits of the row norms
+    o.sa = align256(oz::S * slice_bytes(nbf, naux));
+    o.rl = o.sa + align256(sizeof(double) * (size_t)nbf * naux);
+    o.bytes = o.rl + sizeof(double) * 2 * (size_t)naux;
     return o;
 }
 
 // C5's slices and the per-column arrays of a call, in job->oz_c
 struct CallLayout {
     int nq;
-    size_t sb2, cn, cb, beta, wmax, bytes;
+    size_t c2, sb1, sb2, cn, cb, beta, wmax, bytes;
 };
 CallLayout call_layout(int nbf, int nbf5) {
     CallLayout o;
     o.nq = (nbf5 + oz::QT - 1) / oz::QT * oz::QT;
     const size_t col = align256(sizeof(double) * (size_t)o.nq);
-    o.sb2 = align256((size_t)oz::SB * nbf5 * ((nbf + oz::KC - 1) / oz::KC * oz::KC));
+    o.c2 = align256((size_t)oz::S * nbf5 * ((nbf + oz::KC - 1) / oz::KC * oz::KC));
+    o.sb1 = 2 * o.c2;
+    o.sb2 = o.sb1 + col;
     o.cn = o.sb2 + col;
     o.cb = o.cn + col;
     o.beta = o.cb + col;
@@ -1020,7 +1050,6 @@ int launch_oz(donof_ctx* ctx, cudaStream_t st, const CUtensorMap& ma, const CUte
     if constexpr (MODE != oz::YSUM) {
         if (P.resident && P.nkc == 1) return launch_one<MODE, 1>(ctx, st, ma, mb, P, grid);
         if (P.resident && P.nkc == 2) return launch_one<MODE, 2>(ctx, st, ma, mb, P, grid);
-        if (P.resident && P.nkc == 3) return launch_one<MODE, 3>(ctx, st, ma, mb, P, grid);
     }
     return launch_one<MODE, 0>(ctx, st, ma, mb, P, grid);
 }
@@ -1034,8 +1063,10 @@ oz::Params base_params(donof_job* job, int nbf5) {
     char* cb = job->oz_c.as<char>();
     oz::Params P{};
     P.nbf = job->nbf; P.nbf5 = nbf5; P.naux = job->naux; P.ldq = ldq_of(nbf5);
-    P.ra = reinterpret_cast<double*>(jb + jl.ra);
+    P.sa = reinterpret_cast<double*>(jb + jl.sa);
     P.RL = reinterpret_cast<double*>(jb + jl.rl);
+    P.RLi = P.RL + job->naux;
+    P.sb1 = reinterpret_cast<double*>(cb + cl.sb1);
     P.sb2 = reinterpret_cast<double*>(cb + cl.sb2);
     P.CN = reinterpret_cast<double*>(cb + cl.cn);
     P.cb = reinterpret_cast<double*>(cb + cl.cb);
@@ -1048,16 +1079,16 @@ oz::Params base_params(donof_job* job, int nbf5) {
 
 // Tiles, ring and CTAs of a product with K = nbf and C5's slices as B (T1, T2):
 // B stays in shared memory where its column tile and at least four A stages fit
-// (nbf <= 384) and every column tile has a CTA, else it streams through two stages.
+// (nbf <= 256) and every column tile has a CTA, else it streams through two stages.
 int shape_c5(donof_ctx* ctx, oz::Params& P, long long rows) {
-    constexpr int stage = oz::SB * oz::BS_BYTES;
+    constexpr int stage = oz::S * oz::BS_BYTES;
     P.nrt = (int)((rows + oz::MT - 1) / oz::MT);
     P.nct = (P.nbf5 + oz::QT - 1) / oz::QT;
     P.nkc = (P.nbf + oz::KC - 1) / oz::KC;
     P.k4_last = (P.nbf - (P.nkc - 1) * oz::KC + 31) / 32;
     const long long units = (long long)P.nrt * P.nct;
     const int grid = (int)(units < ctx_ctas(ctx) ? units : ctx_ctas(ctx));
-    P.resident = P.nkc <= 3 && P.nkc * stage + 4 * oz::A_BYTES <= oz::DATA_BYTES && grid >= P.nct;
+    P.resident = P.nkc <= 2 && P.nkc * stage + 4 * oz::A_BYTES <= oz::DATA_BYTES && grid >= P.nct;
     P.ring_off = (P.resident ? P.nkc : 2) * stage;
     P.ring = (oz::DATA_BYTES - P.ring_off) / oz::A_BYTES;
     if (P.ring > oz::RING_MAX) P.ring = oz::RING_MAX;
@@ -1066,21 +1097,23 @@ int shape_c5(donof_ctx* ctx, oz::Params& P, long long rows) {
 
 // rows x digits of 16-byte groups (C5's slices, W's slices): boxes of 64 rows, every
 // digit, the eight groups of a chunk
-int map_b(donof_job* job, const void* base, int rows, int digits, int chunks, CUtensorMap* m) {
-    cuuint64_t dims[3] = {2 * (cuuint64_t)rows, (cuuint64_t)digits, 8 * (cuuint64_t)chunks};
-    cuuint64_t strides[2] = {16 * (cuuint64_t)rows, 16 * (cuuint64_t)rows * digits};
-    cuuint32_t box[3] = {2 * oz::QT, (cuuint32_t)digits, 8};
+int map_b(donof_job* job, const void* base, int rows, int chunks, CUtensorMap* m) {
+    cuuint64_t dims[3] = {2 * (cuuint64_t)rows, oz::S, 8 * (cuuint64_t)chunks};
+    cuuint64_t strides[2] = {16 * (cuuint64_t)rows, 16 * (cuuint64_t)rows * oz::S};
+    cuuint32_t box[3] = {2 * oz::QT, oz::S, 8};
     return make_tmap_u64_flat(job->ctx, m, base, 3, dims, strides, box);
 }
-int map_c5(donof_job* job, int nbf5, CUtensorMap* m) {
-    return map_b(job, job->oz_c.ptr, nbf5, oz::SB, (job->nbf + oz::KC - 1) / oz::KC, m);
+// C5's truncated (T1) or balanced (T2) slices
+int map_c5(donof_job* job, int nbf5, bool balanced, CUtensorMap* m) {
+    const char* base = job->oz_c.as<char>() + (balanced ? call_layout(job->nbf, nbf5).c2 : 0);
+    return map_b(job, base, nbf5, (job->nbf + oz::KC - 1) / oz::KC, m);
 }
 
 // tmp's slices: T2's A operand (MN-major) and Y's (K-major) share the map: boxes of
 // 128 m, the eight groups of a chunk of (q, l), one digit
 int map_t8(donof_job* job, int nbf5, CUtensorMap* m) {
     const cuuint64_t nbf = job->nbf;
-    cuuint64_t dims[3] = {2 * nbf, 8, (cuuint64_t)oz::SW * chunks_of(nbf5, job->naux)};
+    cuuint64_t dims[3] = {2 * nbf, 8, (cuuint64_t)oz::S * chunks_of(nbf5, job->naux)};
     cuuint64_t strides[2] = {16 * nbf, 128 * nbf};
     cuuint32_t box[3] = {2 * oz::MT, 8, 1};
     return make_tmap_u64_flat(job->ctx, m, job->tmp.ptr, 3, dims, strides, box);
@@ -1096,9 +1129,10 @@ int prep(donof_job* job, cudaStream_t st, const double* C, const double* n, cons
     oz::PrepArgs a{};
     a.C = C; a.n = n; a.cj12 = cj12; a.ck12 = ck12;
     a.nbf = job->nbf; a.nbf5 = nbf5; a.nkc = (job->nbf + oz::KC - 1) / oz::KC;
-    a.sb2 = const_cast<double*>(P.sb2); a.CN = const_cast<double*>(P.CN); a.cb = const_cast<double*>(P.cb);
+    a.sb1 = const_cast<double*>(P.sb1); a.sb2 = const_cast<double*>(P.sb2);
+    a.CN = const_cast<double*>(P.CN); a.cb = const_cast<double*>(P.cb);
     a.beta = const_cast<double*>(P.beta);
-    a.out = job->oz_c.as<int8_t>(); a.wmax = P.wmax;
+    a.c1 = job->oz_c.as<int8_t>(); a.c2 = a.c1 + cl.c2; a.wmax = P.wmax;
     oz::prep_kernel<<<cl.nq, 128, 0, st>>>(a); count_launch();
     DONOF_CUDA(ctx, cudaGetLastError());
     return DONOF_OK;
@@ -1111,12 +1145,12 @@ int t1(donof_job* job, cudaStream_t st, int nbf5, double* out) {
     CUtensorMap ma, mb;
     {   // b's slices: boxes of 128 rows (m, l), the eight groups of a chunk of n, one digit
         const cuuint64_t groups = ldn / 16, tiles = ((cuuint64_t)nbf * naux + oz::MT - 1) / oz::MT;
-        cuuint64_t dims[3] = {2 * oz::MT, groups, tiles * oz::SB};
+        cuuint64_t dims[3] = {2 * oz::MT, groups, tiles * oz::S};
         cuuint64_t strides[2] = {16 * oz::MT, 16 * oz::MT * groups};
         cuuint32_t box[3] = {2 * oz::MT, 8, 1};
         DONOF_CHECK(make_tmap_u64_flat(ctx, &ma, job->oz_b, 3, dims, strides, box));
     }
-    DONOF_CHECK(map_c5(job, nbf5, &mb));
+    DONOF_CHECK(map_c5(job, nbf5, false, &mb));
     oz::Params P = base_params(job, nbf5);
     const int grid = shape_c5(ctx, P, (long long)nbf * naux);
     prof_begin(ctx, st);
@@ -1150,16 +1184,18 @@ int ozaki_build(donof_job* job) {
     void* buf = nullptr;
     DONOF_CHECK(dev_alloc(ctx, &buf, jl.bytes));
     int8_t* slices = static_cast<int8_t*>(buf);
-    double* ra = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.ra);
+    double* sa = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.sa);
     double* RL = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.rl);
-    unsigned long long* rn = reinterpret_cast<unsigned long long*>(RL + naux);
+    double* rn = RL + naux;
     cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaMemsetAsync(rn, 0, sizeof(unsigned long long) * (size_t)naux, st);
+    cudaError_t e = cudaMemsetAsync(rn, 0, sizeof(double) * (size_t)naux, st);
     if (e == cudaSuccess) {
-        oz::row_scale_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(job->b, nbf, (long long)naux, ra, rn); count_launch();
-        oz::split_b_kernel<<<16 * ctx->sm_count, 256, 0, st>>>(job->b, ra, nbf, ldn_of(nbf), (long long)naux, slices);
+        oz::row_scale_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(job->b, nbf, (long long)naux, sa,
+                                                               reinterpret_cast<unsigned long long*>(rn));
         count_launch();
-        oz::row_finish_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(nbf, (long long)naux, rn, RL, ra); count_launch();
+        oz::split_b_kernel<<<16 * ctx->sm_count, 256, 0, st>>>(job->b, sa, nbf, ldn_of(nbf), (long long)naux, slices);
+        count_launch();
+        oz::row_finish_kernel<<<(naux + 255) / 256, 256, 0, st>>>((long long)naux, RL, rn); count_launch();
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1194,14 +1230,14 @@ int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const dou
                      const double* ck12, int nbf5) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
-    DONOF_CHECK(job->tmp.ensure(ctx, (size_t)oz::SW * nbf * oz::KC * chunks_of(nbf5, naux)));
+    DONOF_CHECK(job->tmp.ensure(ctx, (size_t)oz::S * nbf * oz::KC * chunks_of(nbf5, naux)));
     // b_pq, and its diagonals again behind it
     DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * (nbf5 + 1) * naux));
     DONOF_CHECK(prep(job, st, C, n, cj12, ck12, nbf5));
     DONOF_CHECK(t1(job, st, nbf5, nullptr));
     CUtensorMap ma, mb;
     DONOF_CHECK(map_t8(job, nbf5, &ma));
-    DONOF_CHECK(map_c5(job, nbf5, &mb));
+    DONOF_CHECK(map_c5(job, nbf5, true, &mb));
     oz::Params P = base_params(job, nbf5);
     const int grid = shape_c5(ctx, P, (long long)P.ldq * naux);
     P.out = job->bpq.as<double>();
@@ -1215,12 +1251,10 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
             int nalpha, int nbeta, const double** ypart, int* nparts) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux, ldq = ldq_of(nbf5), nch = chunks_of(nbf5, naux);
-    const size_t wbytes = (size_t)oz::SW * nbf5 * oz::KC * nch;
-    const JobLayout jl = job_layout(nbf, naux);
-    const bool in_job = wbytes <= jl.ra - jl.work;
-    const size_t o_tv = in_job ? 0 : align256(wbytes);
+    const size_t wbytes = (size_t)oz::S * nbf5 * oz::KC * nch;
+    const size_t o_tv = align256(wbytes);
     DONOF_CHECK(job->W.ensure(ctx, o_tv + sizeof(double) * (size_t)nbf5 * naux));
-    int8_t* w8 = in_job ? reinterpret_cast<int8_t*>(static_cast<char*>(job->oz_b) + jl.work) : job->W.as<int8_t>();
+    int8_t* w8 = job->W.as<int8_t>();
     double* tv = reinterpret_cast<double*>(job->W.as<char>() + o_tv);
     oz::Params P = base_params(job, nbf5);
     const double* bpq = job->bpq.as<double>();
@@ -1234,12 +1268,12 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
         long long blocks = (items + 255) / 256;
         if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
         oz::w_digits_kernel<<<(int)blocks, 256, 0, st>>>(bpq, ck12, tv, nbf5, naux, ldq, nch, P.RL, P.CN, P.beta, P.wmax,
-                                                            w8);
+                                                       w8);
         count_launch();
     }
     DONOF_CUDA(ctx, cudaGetLastError());
 
-    constexpr int stage = oz::SW * oz::BS_BYTES;
+    constexpr int stage = oz::S * oz::BS_BYTES;
     P.nrt = (nbf + oz::MT - 1) / oz::MT;
     P.nct = (nbf5 + oz::QT - 1) / oz::QT;
     P.nkc = nch;
@@ -1272,7 +1306,7 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
     P.out = job->part.as<double>();
     CUtensorMap ma, mb;
     DONOF_CHECK(map_t8(job, nbf5, &ma));
-    DONOF_CHECK(map_b(job, w8, nbf5, oz::SW, nch, &mb));
+    DONOF_CHECK(map_b(job, w8, nbf5, nch, &mb));
     const long long units = (long long)tiles * P.nsplit;
     const int grid = (int)(units < ctx_ctas(ctx) ? units : ctx_ctas(ctx));
     DONOF_CHECK(launch_oz<oz::YSUM>(ctx, st, ma, mb, P, grid));

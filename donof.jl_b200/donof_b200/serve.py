@@ -102,7 +102,7 @@ class Result:
 def footprint(nbf: int, naux: int, nbf5: int, precision: str, fp64_tc: bool = False) -> int:
     """Device bytes a job holds while it runs (upper estimate)."""
     b = 8 * nbf * nbf * naux
-    if fp64_tc:  # b's int8 digit slices and workspace (7 bytes per element, rows padded to 16) and row scales
+    if fp64_tc:  # b's seven int8 digit slices (rows padded to 16) and row scales
         b += 7 * nbf * (-(-nbf // 16) * 16) * naux + 8 * nbf * naux
         # tmp and W as 7 digit slices, their rows padded to 16: more than the FP64 arrays for a small nbf5
         b += max(0, 7 * (-(-nbf5 // 16) * 16) - 8 * nbf5) * (nbf + nbf5) * naux

@@ -1,12 +1,13 @@
 """The FP64 form's contractions from int8 digit slices (csrc/ozaki.cu) at the sizes
 where their tiles, chunks and paddings end, against the FP64 oracle.
 
-Tolerance.  b and C5 carry 48 bits below their largest element per row and column
-(6 balanced digits of 8 bits), so |error of tmp| <= nbf 2^-48 max|b_l| max|C5| / F^2
-with F = 0.498; for N(0, 1) b and orthonormal C that is sqrt(nbf) 6e-14 of the
-largest |tmp|.  tmp and W carry 56 bits below bounds a few bits above their largest
-element, and the dropped digit products lie below 2^-56 of the scales: less than the
-first.  Three contractions of nbf <= 400: 3 * 20 * 6e-14 < 4e-12 of the largest element.
+Tolerance.  T1's operands carry 49 bits below a power of two at most twice the largest
+element of the row (column), truncated, and the dropped digit products are of that size
+too: for N(0, 1) b (elements up to 4) and orthonormal C the error of an element of tmp
+is at most sqrt(nbf) 2^-46 from b's digits (sum_n |C| <= sqrt(nbf)) and as much from
+C's.  tmp, W and T2's C5 carry 56 bits below bounds a few bits above their largest
+element, and their dropped products lie below 2^-62 of the scales: less than the first.
+Three contractions of nbf <= 400: 3 * 2 * 20 * 1.4e-14 < 4e-12 of the largest element.
 """
 import numpy as np
 import pytest
@@ -43,10 +44,10 @@ def inputs(nbf, naux, nbeta, ncwo, nopen, seed=0):
     (128, 21, 16, 3, 0),     # one K chunk, one column tile
     (129, 22, 16, 3, 1),     # two K chunks, nbf5 = 65: two column tiles
     (160, 150, 40, 3, 0),    # (q, l) over several chunks, K steps left out of the last n chunk
-    (256, 3, 64, 3, 0),      # nbf5 = nbf
-    (257, 7, 21, 2, 0),      # three K chunks, nbf5 = 63
-    (384, 5, 16, 2, 0),      # the last size with C5 resident
-    (385, 5, 16, 2, 2),      # C5 streamed
+    (256, 3, 64, 3, 0),      # the last size with C5 resident; nbf5 = nbf
+    (257, 7, 21, 2, 0),      # C5 streamed: three K chunks, nbf5 = 63
+    (384, 5, 16, 2, 0),      # the last of them whole
+    (385, 5, 16, 2, 2),      # a fourth
     (40, 2500, 10, 1, 0),    # a long (q, l) range: 625 chunks, more than one exact int32 range
 ])
 def test_contractions_at_tile_edges_match_the_oracle(cuda_ctx, nbf, naux, nbeta, ncwo, nopen):
