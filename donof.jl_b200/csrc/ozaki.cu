@@ -49,14 +49,14 @@
 //
 // Measured on one B200 (us; in brackets T1 alone from digits, T2 and Y as FP64 GEMMs):
 //   nbf / naux / nbf5    T1            T2            W            Y            Lagrangian
-//   256 / 1024 / 64      110 (131)     40 (85)       23 (20)      31 (81)      (orbital step 345 (433))
-//   202 / 974 / 198      268 (470)     318 (761)     144 (186)    234 (841)    1139 (2238)
-//   384 / 1856 / 320     1774 (2049)   1697 (4649)   553 (698)    1399 (6958)  6496 (14355)
-// (the kernels one by one; the Lagrangian in a loop, at the 1.74 GHz of the power cap).
+//   256 / 1024 / 64      106 (131)     40 (85)       19 (20)      33 (81)      (orbital step 328 (434))
+//   202 / 974 / 198      273 (470)     312 (761)     144 (186)    238 (841)    1094 (2235)
+//   384 / 1856 / 320     1753 (2049)   1711 (4649)   548 (698)    1386 (6958)  6283 (14322)
+// (in a loop, the larger two at the 1.74 GHz of the power cap).
 // At nbf5 = 64 T1 is bound by HBM (b's slices in, tmp's out: 587 MB, 91 us at 6.45
 // TB/s); the larger ones by what the MMAs and the TMA need of shared memory (a
 // chunk of Y: 448 KB of operand reads, 168 KB written, 4900 cycles at 128 bytes a
-// cycle; 5200 measured) and, in T1 and T2, by the drain between two rounds.
+// cycle; 5100 measured) and, in T1 and T2, by the drain between two rounds.
 // elag is within 1e-15 of what the FP64 GEMMs make of the same tmp; its error against
 // 64 bits, 7.2e-14 of the norm, is that of T1's truncated digits.
 //
@@ -110,6 +110,7 @@ constexpr int B_EMPTY = B_FULL + B_STAGES;  // +slot (2): streamed B stage consu
 constexpr int ACC_FULL = B_EMPTY + 2;       // accumulators of a round complete: +0 the last, +1 those from 4 on, +2 3..0
 constexpr int GFREE = ACC_FULL + 3;         // +g (NG_MAX): accumulator g drained and zeroed (count EPI_WARPS)
 constexpr int B_END = GFREE + NG_MAX;       // every MMA of the CTA complete
+static_assert((S * BS_BYTES) >> 4 == 4 * ((2 * 16 * S * QT) >> 4), "B stages adjoin");
 static_assert((B_END + 1) * 8 <= OFF_MISC, "barrier area");
 
 enum Mode {
@@ -269,16 +270,18 @@ __device__ __forceinline__ Unit unit_of(const Params& P, int u) {
     return w;
 }
 
-// One elected lane's MMAs of A slice i (stage at descriptor ad) with B slices 0 ..
-// cnt-1 (stage at bd) over nk4 steps of 32 K: accumulators i .. i + cnt - 1, as one
-// MMA of N = 64 cnt or two (7 = 4 + 3, 6 = 3 + 3, 5 = 3 + 2); part 1 the lower of the
-// two, part 2 the upper, 3 both.  `done` (0: none) is the barrier that the commit
-// behind them arrives on.  i and part are constants after unrolling; the branch on
-// nk4 stays outside the elected lane's region, which is straight code (an MMA takes
-// about 80 issue cycles, 92 to execute: what the warp does between them counts).
-template <int MODE>
-__device__ __forceinline__ void issue_slice(int i, int part, uint32_t tmem, uint64_t ad, uint64_t bd, int nk4,
-                                            uint32_t done) {
+// One elected lane's MMAs of A slice i over NCH K chunks (A stages at descriptors ad,
+// B stages one after the other from bd; the last chunk has nk4 steps of 32 K) with B
+// slices 0 .. cnt-1: accumulators i .. i + cnt - 1, as one MMA of N = 64 cnt or two
+// (7 = 4 + 3, 6 = 3 + 3, 5 = 3 + 2); part 1 the lower of the two, part 2 the upper, 3
+// both.  With `commit`, `done` are the barriers that commits behind them arrive on.
+// i and part are constants after unrolling.  The code is kept short as well as straight:
+// it runs once a round beside 16 epilogue warps, and MMAs of 48 to 128 cycles take 100
+// to issue there (46 in a loop of their own).  With a copy for every nk4 T2 took 322 and
+// Y 246 us at nbf = 202 against 312 and 238.
+template <int MODE, int NCH>
+__device__ __forceinline__ void issue_slice(int i, int part, uint32_t tmem, const uint64_t (&ad)[NCH], uint64_t bd,
+                                            int nk4, const uint32_t (&done)[NCH], bool commit) {
     constexpr int NG = accumulators(MODE);
     const int cnt = (NG - i) < S ? (NG - i) : S;
     const int first = cnt <= 4 ? cnt : (cnt + 1) / 2;
@@ -286,32 +289,30 @@ __device__ __forceinline__ void issue_slice(int i, int part, uint32_t tmem, uint
     constexpr uint64_t astep = (MODE == T2 ? 32 * 16 : 2 * 16 * MT) >> 4;
     constexpr uint64_t bstep = (2 * 16 * S * QT) >> 4;
     constexpr uint32_t amn = MODE == T2 ? 1u << 15 : 0u;
-    auto step = [&](int k4) {
-        if (part & 1)
-            umma_i8(tmem + (uint32_t)(i * QT), ad + k4 * astep, bd + k4 * bstep, idesc_i8(MT, QT * first) | amn, 1u);
+    auto step = [&](uint64_t a, uint64_t b) {
+        if (part & 1) umma_i8(tmem + (uint32_t)(i * QT), a, b, idesc_i8(MT, QT * first) | amn, 1u);
         if ((part & 2) && cnt > first)
-            umma_i8(tmem + (uint32_t)((i + first) * QT), ad + k4 * astep, bd + k4 * bstep + (uint64_t)(first * QT),
+            umma_i8(tmem + (uint32_t)((i + first) * QT), a, b + (uint64_t)(first * QT),
                     idesc_i8(MT, QT * (cnt - first)) | amn, 1u);
     };
-    if (nk4 == 4) {
-        if (elect_one()) {
-            step(0); step(1); step(2); step(3);
-            if (done) umma_commit(done);
+    if (elect_one()) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+            const uint64_t a = ad[c], b = bd + (uint64_t)c * (4 * bstep);
+            const int n = c == NCH - 1 ? nk4 : KC / 32;
+            if (c < NCH - 1) {
+#pragma unroll
+                for (int k4 = 0; k4 < KC / 32; ++k4) step(a + k4 * astep, b + k4 * bstep);
+            } else {
+                step(a, b);
+                if (n > 1) step(a + astep, b + bstep);
+                if (n > 2) step(a + 2 * astep, b + 2 * bstep);
+                if (n > 3) step(a + 3 * astep, b + 3 * bstep);
+            }
         }
-    } else if (nk4 == 3) {
-        if (elect_one()) {
-            step(0); step(1); step(2);
-            if (done) umma_commit(done);
-        }
-    } else if (nk4 == 2) {
-        if (elect_one()) {
-            step(0); step(1);
-            if (done) umma_commit(done);
-        }
-    } else {
-        if (elect_one()) {
-            step(0);
-            if (done) umma_commit(done);
+        if (commit) {
+#pragma unroll
+            for (int c = 0; c < NCH; ++c) umma_commit(done[c]);
         }
     }
     __syncwarp();
@@ -335,12 +336,13 @@ __device__ __forceinline__ uint64_t b_desc(uint32_t addr) {
 // store of zeros; its release (GFREE[g]) comes right after, and the FP64
 // arithmetic of the epilogue runs while the next round's MMAs already fill the
 // released columns.
-// With B resident (NKC = its K chunks, 1 or 2) the order is slice-major over the K
-// chunks, and a round ends with slice 0 against B's upper slices (accumulators 6..4),
-// then its lower ones (3..0): accumulator 7 (NG = 8) is complete a slice earlier, 6..4
-// half a slice earlier, so the epilogue drains them while the last MMAs run and the tensor
-// cores do not wait for it between rounds.  With B streamed (NKC = 0) the order is
-// chunk by chunk.
+// A round ends with slice 0 against B's upper slices (accumulators 6..4), then its
+// lower ones (3..0): accumulator 7 (NG = 8) is complete a slice earlier, 6..4 half a
+// slice earlier, so the epilogue drains them while the last MMAs run and the tensor
+// cores do not wait for it between rounds.  With B resident (NKC = its K chunks, 1 or
+// 2) the order is slice-major over the K chunks and a slice's MMAs of both chunks are
+// one block of the elected lane (T1 at nbf = 256: 111 us, 118 chunk by chunk); with B streamed
+// (NKC = 0) it is chunk by chunk.
 template <int MODE, int NKC>
 __global__ void __launch_bounds__(BOUND_THREADS, 1)
 oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params P) {
@@ -489,28 +491,20 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                             for (int g = NG - 1; g >= i; --g) ok = ok && wait(GFREE + g, up);
                         else if (!__all_sync(0xffffffffu, gready))
                             ok = ok && wait(GFREE + i, up);
-                        uint32_t db[NKC];
+                        uint32_t done[NKC];
                         uint64_t da[NKC];
 #pragma unroll
                         for (int kc = 0; kc < NKC; ++kc) {
                             ok = ok && landed();
                             if (!ok) break;
-                            const uint32_t done = fb + 8u * RING_MAX;
-                            const uint64_t d = ad;
+                            done[kc] = fb + 8u * RING_MAX;
+                            da[kc] = ad;
                             next();
-                            if (i > 0 && kc == NKC - 1) gready = mbar_test(bar(GFREE + i - 1), up);
-                            fence_after();
-                            const uint64_t bd = b_desc(sbase + kc * B_BYTES);
-                            const int nk4 = kc == NKC - 1 ? P.k4_last : KC / 32;
-                            if (i > 0) {
-                                issue_slice<MODE>(i, 3, tmem, d, bd, nk4, done);
-                            } else {
-                                issue_slice<MODE>(0, 2, tmem, d, bd, nk4, 0);
-                                db[kc] = done;
-                                da[kc] = d;
-                            }
                         }
                         if (!ok) break;
+                        if (i > 0) gready = mbar_test(bar(GFREE + i - 1), up);
+                        fence_after();
+                        issue_slice<MODE, NKC>(i, i > 0 ? 3 : 2, tmem, da, b_desc(sbase), P.k4_last, done, i > 0);
                         if (i == NG - S) {  // slice 1 (NG = 8) or the upper part of slice 0: the last accumulator
                             if (elect_one()) umma_commit(bar(ACC_FULL));
                             __syncwarp();
@@ -518,41 +512,51 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                         if (i == 0) {
                             if (elect_one()) umma_commit(bar(ACC_FULL + 1));
                             __syncwarp();
-#pragma unroll
-                            for (int kc = 0; kc < NKC; ++kc)
-                                issue_slice<MODE>(0, 1, tmem, da[kc], b_desc(sbase + kc * B_BYTES),
-                                                      kc == NKC - 1 ? P.k4_last : KC / 32, db[kc]);
+                            issue_slice<MODE, NKC>(0, 1, tmem, da, b_desc(sbase), P.k4_last, done, true);
                             if (elect_one()) umma_commit(bar(ACC_FULL + 2));
                             __syncwarp();
                         }
                     }
                 } else {
                     const Unit w = unit_of<MODE, resident>(P, u);
-                    for (int g = NG - 1; g >= 0; --g) ok = ok && wait(GFREE + g, up);
-                    for (int kc = w.c0; kc < w.c0 + w.nc && ok; ++kc, ++bs) {
+                    const int end = w.c0 + w.nc;
+                    for (int kc = w.c0; kc < end && ok; ++kc, ++bs) {
                         const int slot = bs & 1;
                         const uint64_t bd = b_desc(sbase + slot * B_BYTES);
                         const int nk4 = kc == P.nkc - 1 ? P.k4_last : KC / 32;
                         ok = wait(B_FULL + slot, (uint32_t)((bs >> 1) & 1));
 #pragma unroll
                         for (int ii = 0; ii < S; ++ii) {
+                            const int i = S - 1 - ii;
+                            if (kc == w.c0)
+                                for (int g = ii == 0 ? NG - 1 : i; g >= i; --g) ok = ok && wait(GFREE + g, up);
                             ok = ok && landed();
                             if (!ok) break;
-                            const uint32_t done = fb + 8u * RING_MAX;
-                            const uint64_t d = ad;
+                            const uint32_t done[1] = {fb + 8u * RING_MAX};
+                            const uint64_t da[1] = {ad};
                             next();
                             fence_after();
-                            issue_slice<MODE>(S - 1 - ii, 3, tmem, d, bd, nk4, done);
+                            if (i == 0 && kc == end - 1) {
+                                issue_slice<MODE, 1>(0, 2, tmem, da, bd, nk4, done, false);
+                                if (elect_one()) {
+                                    if (NG == S) umma_commit(bar(ACC_FULL));
+                                    umma_commit(bar(ACC_FULL + 1));
+                                }
+                                __syncwarp();
+                                issue_slice<MODE, 1>(0, 1, tmem, da, bd, nk4, done, true);
+                                if (elect_one()) umma_commit(bar(ACC_FULL + 2));
+                                __syncwarp();
+                            } else {
+                                issue_slice<MODE, 1>(i, 3, tmem, da, bd, nk4, done, true);
+                                if (NG > S && i == NG - S && kc == end - 1) {
+                                    if (elect_one()) umma_commit(bar(ACC_FULL));
+                                    __syncwarp();
+                                }
+                            }
                         }
                         if (ok && elect_one()) umma_commit(bar(B_EMPTY + slot));
                         __syncwarp();
                     }
-                    if (ok && elect_one()) {
-                        umma_commit(bar(ACC_FULL));
-                        umma_commit(bar(ACC_FULL + 1));
-                        umma_commit(bar(ACC_FULL + 2));
-                    }
-                    __syncwarp();
                 }
             }
             if (elect_one()) umma_commit(bar(B_END));
