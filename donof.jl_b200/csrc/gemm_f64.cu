@@ -82,6 +82,13 @@ cudaError_t launch_layout(const GemmF64Args& p, bool ak, bool bk, bool vec, cuda
     return launch_vec<BM, BN, WM, WN, false, false>(p, vec, st, persistent);
 }
 
+// The narrow tiles (one CTA per tile, B K-contiguous)
+template <int BM, int BN, int WM>
+cudaError_t launch_narrow(const GemmF64Args& p, bool ak, bool vec, cudaStream_t st) {
+    return ak ? launch_vec<BM, BN, WM, 1, true, true>(p, vec, st, false)
+              : launch_vec<BM, BN, WM, 1, false, true>(p, vec, st, false);
+}
+
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <int BM, int BN, int WM, int WN, bool AK, bool BKM, bool VEC, bool LOOP>
@@ -192,6 +199,10 @@ int gemm_f64_run(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajor, 
         e = launch_layout<64, 64, 2, 2>(p, a_kmajor, b_kmajor, vec, st, persistent);
     else if (tile == GemmTile::SmallW8)
         e = launch_layout<64, 64, 2, 4>(p, a_kmajor, b_kmajor, vec, st, persistent);
+    else if (tile == GemmTile::N24 && b_kmajor)
+        e = launch_narrow<48, 24, 3>(p, a_kmajor, vec, st);
+    else if (tile == GemmTile::N40 && b_kmajor)
+        e = launch_narrow<32, 40, 2>(p, a_kmajor, vec, st);
     else
         e = launch_layout<32, 32, 2, 2>(p, a_kmajor, b_kmajor, vec, st, persistent);
     if (e != cudaSuccess) {
@@ -328,6 +339,26 @@ constexpr int kNT = 4;
 const GemmTile kTiles[kNT] = {GemmTile::Large, GemmTile::Small, GemmTile::Tiny, GemmTile::SmallW8};
 const int kTileBM[kNT] = {128, 64, 32, 64}, kTileBN[kNT] = {64, 64, 32, 64};
 
+// The narrow tiles worth timing for an M x N result: those that pad it to less than
+// 32 x 32 tiles do (66 columns are 72 or 80 instead of 96, 80 are 80).  At equal padding
+// they lose (T1 at 96 x 96 x 96, 464 products: 35 and 31 us against 33; 192 x 160 x 192,
+// 928 products: 387 and 371 against 353); with less they gain (91 x 66 x 91, 437
+// products: 29 and 31 us against 35; 96 x 80 x 96, 464 products: 31 us against 33).
+int narrow_tiles(bool b_kmajor, int M, int N, GemmTile (&tiles)[2], int (&bm)[2], int (&bn)[2]) {
+    if (!b_kmajor) return 0;
+    auto padded = [&](int tm, int tn) { return (long long)((M + tm - 1) / tm * tm) * ((N + tn - 1) / tn * tn); };
+    int n = 0;
+    auto add = [&](GemmTile t, int tm, int tn) {
+        if (padded(tm, tn) >= padded(32, 32)) return;
+        tiles[n] = t;
+        bm[n] = tm;
+        bn[n++] = tn;
+    };
+    add(GemmTile::N24, 48, 24);
+    add(GemmTile::N40, 32, 40);
+    return n;
+}
+
 }  // namespace
 
 int gemm_f64_tuned(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajor, const GemmF64Args& p,
@@ -339,12 +370,19 @@ int gemm_f64_tuned(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajor
     TuneVal v;
     if (tune_lookup(key, &v)) return gemm_f64_run(ctx, st, a_kmajor, b_kmajor, p, v.tile, v.persistent);
     if (capturing(st)) return gemm_f64(ctx, st, a_kmajor, b_kmajor, p, heuristic);
-    // every tile shape, one CTA per tile and persistent
-    const int best = time_candidates(ctx, st, 2 * kNT, [&](int c) {
-        return gemm_f64_run(ctx, st, a_kmajor, b_kmajor, p, kTiles[c % kNT], c >= kNT);
+    // every tile shape, one CTA per tile and persistent, then the narrow ones
+    GemmTile narrow[2];
+    int bm[2], bn[2];
+    const int nn = narrow_tiles(b_kmajor, p.M, p.N, narrow, bm, bn);
+    auto choice = [&](int c) {
+        return c < 2 * kNT ? TuneVal{kTiles[c % kNT], 1, c >= kNT} : TuneVal{narrow[c - 2 * kNT], 1, false};
+    };
+    const int best = time_candidates(ctx, st, 2 * kNT + nn, [&](int c) {
+        const TuneVal t = choice(c);
+        return gemm_f64_run(ctx, st, a_kmajor, b_kmajor, p, t.tile, t.persistent);
     });
     if (best < 0) return DONOF_ERR_CUDA;
-    tune_store(key, TuneVal{kTiles[best % kNT], 1, best >= kNT});
+    tune_store(key, choice(best));
     return DONOF_OK;  // every candidate wrote the same C
 }
 
@@ -361,26 +399,33 @@ int partials_choice(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajo
     p.M = M; p.N = N; p.K = K;
     p.A = A; p.lda = lda; p.B = B; p.ldb = ldb;
     p.alpha = 1.0; p.beta = 0.0; p.batch = 1; p.splits = 1; p.kchunk = K;
-    // candidates: each tile shape with about one and about two CTAs per SM
+    // candidates: each tile shape with about one and about two CTAs per SM, the small
+    // tiles, of which six to eight fit, with up to four
     std::vector<TuneVal> cands;
     {
         int sp = 1;
         const GemmTile h = pick_tile(ctx, M, N, K, true, &sp);
         cands.push_back(TuneVal{h, sp});
         const int max_splits = K / 64 > 1 ? K / 64 : 1;
-        for (int t = 0; t < kNT; ++t) {
-            const long long tiles = (long long)((M + kTileBM[t] - 1) / kTileBM[t]) * ((N + kTileBN[t] - 1) / kTileBN[t]);
-            for (int f = 1; f <= 2; ++f) {
+        auto add = [&](GemmTile tile, int bm, int bn) {
+            const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+            const int most = bm * bn <= 32 * 40 ? 4 : 2;
+            for (int f = 1; f <= most; ++f) {
                 long long s = (f * (long long)ctx->sm_count + tiles - 1) / tiles;
                 if (s > max_splits) s = max_splits;
                 if (s < 1) s = 1;
                 bool dup = false;
-                for (const TuneVal& c : cands) dup = dup || (c.tile == kTiles[t] && c.splits == (int)s);
-                if (!dup) cands.push_back(TuneVal{kTiles[t], (int)s});
+                for (const TuneVal& c : cands) dup = dup || (c.tile == tile && c.splits == (int)s);
+                if (!dup) cands.push_back(TuneVal{tile, (int)s});
             }
-        }
+        };
+        for (int t = 0; t < kNT; ++t) add(kTiles[t], kTileBM[t], kTileBN[t]);
         const size_t nplain = cands.size();
         for (size_t c = 0; c < nplain; ++c) cands.push_back(TuneVal{cands[c].tile, cands[c].splits, true});
+        GemmTile narrow[2];
+        int bm[2], bn[2];
+        const int nn = narrow_tiles(b_kmajor, M, N, narrow, bm, bn);
+        for (int t = 0; t < nn; ++t) add(narrow[t], bm[t], bn[t]);
     }
     auto config = [&](const TuneVal& c, GemmF64Args* q, int* ns) {
         *q = p;

@@ -12,7 +12,10 @@ namespace donof {
 
 // Tile shapes of the FP64 GEMM.  SmallW8 (64 x 64 over 8 warps of 32 x 16):
 // more warps per SM for short-K products.
-enum class GemmTile { Large /*128x64*/, Small /*64x64*/, Tiny /*32x32*/, SmallW8 /*64x64, 8 warps*/ };
+enum class GemmTile {
+    Large /*128x64*/, Small /*64x64*/, Tiny /*32x32*/, SmallW8 /*64x64, 8 warps*/,
+    N24 /*48x24, 3 warps*/, N40 /*32x40, 2 warps; both with a K-contiguous B only*/
+};
 
 // C = alpha*op(A)op(B) + beta*C on stream st (see gemm_f64.cuh for addressing).
 int gemm_f64(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajor, GemmF64Args p,
