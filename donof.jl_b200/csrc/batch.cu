@@ -717,7 +717,7 @@ int donof_batch_create(donof_ctx* ctx, int count, const donof_batch_shape* shape
     field(off_bpq, [](const S& h) { return (size_t)h.nbf5 * h.nbf5 * h.naux; });
     field(off_W, [](const S& h) { return (size_t)h.nbf5 * h.nbf5 * h.naux; });
     field(off_tv, [](const S& h) { return (size_t)h.nbf5 * h.naux; });
-    field(off_tw, [](const S& h) { return (size_t)3 * h.nbf * h.nbf5; });
+    field(off_tw, [](const S& h) { return (size_t)2 * h.nbf * h.nbf5; });
     field(off_rw, [](const S& h) { return rotate_work_doubles(h.nbf); });
     int rc = B->arena.ensure(ctx, sizeof(double) * acc);
     if (rc != DONOF_OK) {

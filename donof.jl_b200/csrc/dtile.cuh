@@ -30,9 +30,10 @@ constexpr int APANEL = (KC * AS > TM * ATS) ? KC * AS : TM * ATS;  // doubles of
 
 // Shared memory (doubles) of one tile product with TN output columns: the ring
 // of A and B panels, which also holds the final cross-warp sum.
-template <int TN>
+template <int TN, bool DUAL = false>
 constexpr int smem_doubles() {
-    return (NBUF * (APANEL + TN * BS) > THREADS * TN) ? NBUF * (APANEL + TN * BS) : THREADS * TN;
+    constexpr int ring = NBUF * (APANEL + (DUAL ? 2 : 1) * TN * BS);
+    return ring > THREADS * TN ? ring : THREADS * TN;
 }
 
 // C(i, j) for i < M, j < N of one GEMM: C = alpha opA(A) opB(B) (+ C when accumulate)
@@ -50,6 +51,10 @@ struct Gemm {
     int M, N, K;
     double alpha;
     bool accumulate;
+    // DUAL tiles: opB(k, j) = B(k, j) bscale[j] + B2(k, j), formed from the staged panels
+    // as the fragments are read (B2 with B's strides, B not transposed)
+    const double* B2 = nullptr;
+    const double* bscale = nullptr;
 };
 
 template <int TN>
@@ -77,7 +82,7 @@ __device__ __forceinline__ int aoff(int i, int k) { return TA ? i * ATS + k : k 
 // Stage the K panel [k0, k0 + KC) of the tile (i0, j0) into the A and B panel
 // buffers (zeros outside the matrices) as one cp.async group; the general
 // path, used at the edges of the matrices and for unaligned operands.
-template <int TN, bool TA>
+template <int TN, bool TA, bool DUAL>
 __device__ __forceinline__ void load_panel(const Gemm& g, int i0, int j0, int k0, double* As, double* Bs) {
     const int tid = threadIdx.x;
     for (int e = tid; e < TM * KC; e += THREADS) {
@@ -101,6 +106,10 @@ __device__ __forceinline__ void load_panel(const Gemm& g, int i0, int j0, int k0
             cp_async8(dst, g.tb ? g.B + gj + (long long)gk * g.ldb : g.B + gk + (long long)gj * g.ldb);
         else
             *dst = 0.0;
+        if (DUAL) {
+            if (gj < g.N && gk < g.K) cp_async8(dst + TN * BS, g.B2 + gk + (long long)gj * g.ldb);
+            else dst[TN * BS] = 0.0;
+        }
     }
     cp_async_commit();
 }
@@ -111,7 +120,7 @@ __device__ __forceinline__ void load_panel(const Gemm& g, int i0, int j0, int k0
 // doubles, contiguous in memory and in the panel, at fixed strides in every
 // panel.  Everything else, and the last panel when K is not a multiple of KC,
 // goes through load_panel.
-template <int TN, bool TA>
+template <int TN, bool TA, bool DUAL>
 struct PanelLoader {
     // A as stored: pairs (i, i+1) along a k row; transposed A: pairs (k, k+1) along a row i
     static constexpr int APER = TA ? KC / 2 : TM / 2;           // pairs per line
@@ -125,12 +134,14 @@ struct PanelLoader {
     long long a_line;     // A elements between two lines copied by this thread
     long long a_panel;    // A elements between panels
     long long b_jstep;    // B elements between two columns copied by this thread
+    long long b_second;   // DUAL: from B to B2
     int a_dst, b_dst;     // offsets in the panel buffers
 
     __device__ __forceinline__ PanelLoader(const Gemm& g, int i0, int j0) {
         const int tid = threadIdx.x;
         fast = !g.tb && (g.lda & 1) == 0 && (g.ldb & 1) == 0 &&
                ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) == 0 &&
+               (!DUAL || (reinterpret_cast<uintptr_t>(g.B2) & 15) == 0) &&
                i0 + TM <= g.M && j0 + TN <= g.N;
         const int ap = 2 * (tid % APER), al = tid / APER;  // pair offset within the line, line
         if (TA) {  // line = row i (k contiguous)
@@ -147,6 +158,7 @@ struct PanelLoader {
         b_src = g.B + bk + (long long)(j0 + bj) * g.ldb;
         b_jstep = (long long)BJSTEP * g.ldb;
         b_dst = bj * BS + bk;
+        b_second = DUAL ? g.B2 - g.B : 0;
     }
 
     __device__ __forceinline__ void load(const Gemm& g, int i0, int j0, int p, double* As, double* Bs) const {
@@ -157,10 +169,13 @@ struct PanelLoader {
 #pragma unroll
             for (int r = 0; r < APASS; ++r) cp_async16(As + a_dst + r * ADST, sa + r * a_line);
 #pragma unroll
-            for (int r = 0; r < TN / BJSTEP; ++r) cp_async16(Bs + b_dst + r * BJSTEP * BS, sb + r * b_jstep);
+            for (int r = 0; r < TN / BJSTEP; ++r) {
+                cp_async16(Bs + b_dst + r * BJSTEP * BS, sb + r * b_jstep);
+                if (DUAL) cp_async16(Bs + TN * BS + b_dst + r * BJSTEP * BS, sb + r * b_jstep + b_second);
+            }
             cp_async_commit();
         } else {
-            load_panel<TN, TA>(g, i0, j0, p * KC, As, Bs);
+            load_panel<TN, TA, DUAL>(g, i0, j0, p * KC, As, Bs);
         }
     }
 };
@@ -169,7 +184,7 @@ struct PanelLoader {
 // tile grid) with A read as stored (TA = false) or transposed (TA = true; must
 // equal g.ta).  sm holds smem_doubles<TN>() doubles.  The caller's CTA has
 // THREADS threads; every thread must call this.
-template <int TN, bool TA>
+template <int TN, bool TA, bool DUAL = false>
 __device__ void tile_t(const Gemm& g, int t, double* sm) {
     static_assert(TN == 16 || TN == 32, "tile width");
     constexpr int NI = TN / 8;      // n8 blocks
@@ -187,11 +202,16 @@ __device__ void tile_t(const Gemm& g, int t, double* sm) {
         for (int b = 0; b < NI; ++b)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[a][b][e] = 0.0;
-    auto As = [&](int buf) { return sm + buf * (APANEL + TN * BS); };
-    auto Bs = [&](int buf) { return sm + buf * (APANEL + TN * BS) + APANEL; };
+    constexpr int BUF = APANEL + (DUAL ? 2 : 1) * TN * BS;
+    auto As = [&](int buf) { return sm + buf * BUF; };
+    auto Bs = [&](int buf) { return sm + buf * BUF + APANEL; };
+    double bscale[NI];
+#pragma unroll
+    for (int ni = 0; ni < NI; ++ni)
+        bscale[ni] = DUAL && j0 + ni * 8 + gq < g.N ? g.bscale[j0 + ni * 8 + gq] : 0.0;
 
     const int npan = (g.K + KC - 1) / KC;
-    const PanelLoader<TN, TA> ld(g, i0, j0);
+    const PanelLoader<TN, TA, DUAL> ld(g, i0, j0);
     __syncthreads();  // the buffers may still be read by the previous tile
     // prologue: the first NBUF - 1 panels in flight (one commit group each, empty ones too)
 #pragma unroll
@@ -218,7 +238,10 @@ __device__ void tile_t(const Gemm& g, int t, double* sm) {
                 af[mi][1] = A_[aoff<TA>(mi * 16 + gq + 8, kk + tq)];
             }
 #pragma unroll
-            for (int ni = 0; ni < NI; ++ni) bf[ni] = B_[(ni * 8 + gq) * BS + kk + tq];
+            for (int ni = 0; ni < NI; ++ni) {
+                const double* b = B_ + (ni * 8 + gq) * BS + kk + tq;
+                bf[ni] = DUAL ? fma(b[0], bscale[ni], b[TN * BS]) : b[0];
+            }
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi)
 #pragma unroll

@@ -204,7 +204,7 @@ struct TailJob {
     const void* part;  // Y partials: part[g * pstride + m + nbf * b], g < nparts
     long long pstride;
     double *Hmat, *elag, *E;
-    double* work;  // 3 * nbf * nbf5 doubles
+    double* work;  // 2 * nbf * nbf5 doubles
     void* state;
     const int* skip;
     int nbf, nbf5, part_f32, nparts, cta0, ctas;

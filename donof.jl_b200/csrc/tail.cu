@@ -10,9 +10,12 @@
 //   E_elec = sum_{i < nbf5} elag[i, i] + n_i H_mat[i, i]
 //
 // Stage 1 runs the HC tiles and the reduction of the Y partials side by side,
-// stage 2 forms Bp, stage 3 the H_mat and elag tiles; the last CTA to finish
-// stage 3 sums the energy in a fixed order.  Bounded grid barriers separate
-// the stages.
+// stage 2 the H_mat and elag tiles; the last CTA to finish it sums the energy in
+// a fixed order.  A bounded grid barrier separates the stages.  What bounds the
+// tail is latency (the barrier, loads of what other SMs wrote, a launch), not its
+// FLOPs: Bp is formed from the staged HC and Y panels as elag's tiles read them,
+// instead of in a stage of its own behind a second barrier (8.2 against 9.9 us at nbf =
+// 24, 11.4 against 13.4 at 91, 15 against 17 at 256 x 64).
 #include <atomic>
 #include "dtile.cuh"
 #include "kernels.cuh"
@@ -38,7 +41,7 @@ struct TailArgs {
     int part_f32;
     int nparts;
     long long pstride;
-    double *Y, *HC, *Bp;  // scratch, nbf x nbf5 each
+    double *Y, *HC;  // scratch, nbf x nbf5 each
     double *Hmat, *elag, *E;
     TailState* ts;
     dtile::WaitCtl wc;
@@ -150,12 +153,7 @@ __device__ __forceinline__ void tail_body(const TailArgs& a, int cta, int G, dou
     }
     if (!dtile::grid_barrier(gs, epoch, G, a.wc)) return;
 
-    // ---- stage 2: Bp = HC diag(n) + Y
-    for (long long i = (long long)cta * dtile::THREADS + tid; i < ny; i += (long long)G * dtile::THREADS)
-        a.Bp[i] = a.HC[i] * a.n[i / nbf] + a.Y[i];
-    if (!dtile::grid_barrier(gs, epoch, G, a.wc)) return;
-
-    // ---- stage 3: H_mat = C^T HC, elag[:, :nbf5] = C^T Bp
+    // ---- stage 2: H_mat = C^T HC, elag[:, :nbf5] = C^T (HC diag(n) + Y)
     dtile::Gemm gh;
     gh.A = a.C; gh.lda = nbf; gh.ta = true;
     gh.B = a.HC; gh.ldb = nbf; gh.tb = false;
@@ -163,12 +161,13 @@ __device__ __forceinline__ void tail_body(const TailArgs& a, int cta, int G, dou
     gh.M = nbf; gh.N = nbf5; gh.K = nbf;
     gh.alpha = 1.0; gh.accumulate = false;
     dtile::Gemm ge = gh;
-    ge.B = a.Bp;
+    ge.B2 = a.Y;
+    ge.bscale = a.n;
     ge.C = a.elag;
     const int nt = dtile::tiles<TL_TN>(gh);
     for (int w = cta; w < 2 * nt; w += G) {
         if (w < nt) dtile::tile<TL_TN>(gh, w, sm);
-        else dtile::tile<TL_TN>(ge, w - nt, sm);
+        else dtile::tile_t<TL_TN, true, true>(ge, w - nt, sm);
     }
     if (a.E == nullptr) return;
     // ---- energy: the last CTA to finish sums the diagonals in a fixed order
@@ -222,7 +221,7 @@ __global__ void __launch_bounds__(dtile::THREADS) tail_grouped_kernel(const Tail
         a.nbf = t.nbf; a.nbf5 = t.nbf5;
         a.part = t.part; a.part_f32 = t.part_f32; a.nparts = t.nparts; a.pstride = t.pstride;
         a.ts = static_cast<TailState*>(t.state);
-        a.Y = t.work; a.HC = a.Y + ny; a.Bp = a.HC + ny;
+        a.Y = t.work; a.HC = a.Y + ny;
         a.Hmat = t.Hmat; a.elag = t.elag; a.E = t.E;
         a.wc = wc;
         tail_body(a, cta - c0, cn, sm);
@@ -233,7 +232,7 @@ __global__ void __launch_bounds__(dtile::THREADS) tail_grouped_kernel(const Tail
 }  // namespace
 
 int tail_grouped(donof_ctx* ctx, cudaStream_t st, const TailJob* jobs, int njobs, void* states, int grid) {
-    const int smem = (int)sizeof(double) * dtile::smem_doubles<TL_TN>();
+    const int smem = (int)sizeof(double) * dtile::smem_doubles<TL_TN, true>();
     static std::atomic<unsigned long long> attr_mask{0};
     const unsigned long long bit = 1ull << (ctx->device & 63);
     if (!(attr_mask.load(std::memory_order_acquire) & bit)) {
@@ -266,7 +265,7 @@ int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf;
     const size_t ny = (size_t)nbf * nbf5;
-    DONOF_CHECK(job->small.ensure(ctx, 256 + sizeof(double) * 3 * ny));
+    DONOF_CHECK(job->small.ensure(ctx, 256 + sizeof(double) * 2 * ny));
     char* base = job->small.as<char>();
     TailArgs a{};
     a.C = C; a.H = H; a.n = n;
@@ -275,10 +274,9 @@ int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double
     a.ts = reinterpret_cast<TailState*>(base);
     a.Y = reinterpret_cast<double*>(base + 256);
     a.HC = a.Y + ny;
-    a.Bp = a.HC + ny;
     a.Hmat = Hmat; a.elag = elag; a.E = E;
     a.wc = dtile::wait_ctl(ctx);
-    const int smem = (int)sizeof(double) * dtile::smem_doubles<TL_TN>();
+    const int smem = (int)sizeof(double) * dtile::smem_doubles<TL_TN, true>();
     static std::atomic<unsigned long long> attr_mask{0};
     const unsigned long long bit = 1ull << (ctx->device & 63);
     if (!(attr_mask.load(std::memory_order_acquire) & bit)) {
