@@ -73,9 +73,18 @@ int gemm_f64_partials_splits(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, boo
 // Fused FP64 tail of the Lagrangian (tail.cu): Y = sum of nparts partials
 // (FP32 or FP64, part[g * pstride + m + nbf * b]), HC = H C5, H_mat = C^T HC,
 // elag = [n o H_mat + C^T Y | 0] and E_elec (when E != nullptr).
+// The tail's barrier state: tail_state returns its TAIL_STATE_WORDS words (in job->small,
+// sized for the tail), which a kernel that runs earlier in the call zeroes with
+// zero_tail_state; elag_tail_f64 is then told so and needs no memset of its own.
+constexpr int TAIL_STATE_WORDS = 8;
+int tail_state(donof_job* job, int nbf5, unsigned** words);
+__device__ __forceinline__ void zero_tail_state(unsigned* words) {
+    if (words != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < TAIL_STATE_WORDS)
+        words[threadIdx.x] = 0;
+}
 int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double* H, const double* n, int nbf5,
                   const void* part, bool part_f32, int nparts, long long pstride, double* Hmat, double* elag,
-                  double* E);
+                  double* E, bool state_zeroed = false);
 
 // Eigenvalues w and eigenvectors V (columns) of Symmetric(G) on the device by
 // the parallel block Jacobi method (eigh.cu): A and V hold N x N with N =
@@ -106,7 +115,7 @@ int t1_ozaki(donof_job* job, cudaStream_t st, const double* C, int nbf5, double*
 int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
                      const double* ck12, int nbf5);
 int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12, const double* ck12, int nbf5,
-            int nalpha, int nbeta, const double** ypart, int* nparts);
+            int nalpha, int nbeta, const double** ypart, int* nparts, unsigned* tail_words);
 
 // Tensor maps with zero fill (mixed.cu): 128-byte swizzle, or none (u64_flat)
 int make_tmap_u64_flat(donof_ctx* ctx, CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,

@@ -32,7 +32,9 @@ namespace {
 // wbuild::LT aux indices, one tile per CTA step (b need not be symmetric).
 __global__ void __launch_bounds__(256) w_diag_kernel(const double* __restrict__ bpq, const double* __restrict__ n,
                                                      const double* __restrict__ cj12, int nbf5, int naux, int nalpha,
-                                                     int nbeta, double* __restrict__ tv) {
+                                                     int nbeta, double* __restrict__ tv,
+                                                     unsigned* tail_words) {
+    zero_tail_state(tail_words);
     __shared__ double sd[wbuild::DIAG_SM];
     const long long units = wbuild::diag_units(nbf5, naux);
     for (long long u = blockIdx.x; u < units; u += gridDim.x)
@@ -58,7 +60,9 @@ __global__ void __launch_bounds__(256, 4) build_w_fused_kernel(const double* __r
                                                             const double* __restrict__ n,
                                                             const double* __restrict__ cj12,
                                                             const double* __restrict__ ck12, int nbf5, int naux,
-                                                            int nalpha, int nbeta, double* __restrict__ W) {
+                                                            int nalpha, int nbeta, double* __restrict__ W,
+                                                            unsigned* tail_words) {
+    zero_tail_state(tail_words);
     __shared__ double tb[wbuild::LT][32][33];
     __shared__ double sd[wbuild::LT * FUSED_W_MAX];
     __shared__ double stv[wbuild::LT][32];
@@ -178,17 +182,20 @@ __global__ void hcore_kernel(const double* __restrict__ C, const double* __restr
 // W of every aux index into W (Kt * nbf5 values; W + Kt * nbf5 holds the Kt
 // diagonal terms when they are built in a pass of their own).
 int build_w(donof_ctx* ctx, cudaStream_t st, const double* bpq, const double* n, const double* cj12,
-            const double* ck12, int nbf5, int naux, int nalpha, int nbeta, double* W) {
+            const double* ck12, int nbf5, int naux, int nalpha, int nbeta, double* W,
+            unsigned* tail_words) {
     long long blocks = wbuild::tiles(nbf5, naux);
     if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
     if (nbf5 <= FUSED_W_MAX) {
-        build_w_fused_kernel<<<(int)blocks, 256, 0, st>>>(bpq, n, cj12, ck12, nbf5, naux, nalpha, nbeta, W);
+        build_w_fused_kernel<<<(int)blocks, 256, 0, st>>>(bpq, n, cj12, ck12, nbf5, naux, nalpha, nbeta, W,
+                                                        tail_words);
         count_launch();
     } else {
         double* tv = W + (size_t)nbf5 * naux * nbf5;  // n'_b d_b^l + t_b^l (Kt values)
         long long dblocks = wbuild::diag_units(nbf5, naux);
         if (dblocks > 8LL * ctx->sm_count) dblocks = 8LL * ctx->sm_count;
-        w_diag_kernel<<<(int)dblocks, 256, 0, st>>>(bpq, n, cj12, nbf5, naux, nalpha, nbeta, tv); count_launch();
+        w_diag_kernel<<<(int)dblocks, 256, 0, st>>>(bpq, n, cj12, nbf5, naux, nalpha, nbeta, tv, tail_words);
+        count_launch();
         build_w_kernel<<<(int)blocks, 256, 0, st>>>(bpq, ck12, tv, nbf5, naux, W); count_launch();
     }
     DONOF_CUDA(ctx, cudaGetLastError());
@@ -242,20 +249,22 @@ namespace {
 
 // Y = sum_{q,l} tmp[m, q + nbf5*l] W[q + nbf5*l, b], left as FP64 partials
 // (nbf x nbf5 each): the transforms, W and the split-K product, on the FP64 GEMM
-// or from digit slices on the tensor cores.
+// or from digit slices on the tensor cores.  W's kernels zero the tail's barrier state.
 int y_partials(donof_job* job, cudaStream_t st, const double* C, const double* n, const double* cj12,
                const double* ck12, int nbf5, int nalpha, int nbeta, const double** ypart, int* nparts) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
+    unsigned* words = nullptr;
+    DONOF_CHECK(tail_state(job, nbf5, &words));
     if (job->oz_b) {
         DONOF_CHECK(transforms_ozaki(job, st, C, n, cj12, ck12, nbf5));
-        return y_ozaki(job, st, n, cj12, ck12, nbf5, nalpha, nbeta, ypart, nparts);
+        return y_ozaki(job, st, n, cj12, ck12, nbf5, nalpha, nbeta, ypart, nparts, words);
     }
     const long long Kt = (long long)nbf5 * naux;
     DONOF_CHECK(transforms_f64(job, st, C, nbf5));
     DONOF_CHECK(job->W.ensure(ctx, sizeof(double) * (size_t)Kt * (nbf5 + 1)));
     double* W = job->W.as<double>();
-    DONOF_CHECK(build_w(ctx, st, job->bpq.as<double>(), n, cj12, ck12, nbf5, naux, nalpha, nbeta, W));
+    DONOF_CHECK(build_w(ctx, st, job->bpq.as<double>(), n, cj12, ck12, nbf5, naux, nalpha, nbeta, W, words));
     return gemm_f64_partials(ctx, st, false, true, nbf, nbf5, (int)Kt, job->tmp.as<double>(), nbf, W, Kt, &job->part,
                              ypart, nparts);
 }
@@ -270,7 +279,7 @@ int lagrange2_f64(donof_job* job, cudaStream_t st, const double* C, const double
     int nparts = 1;
     DONOF_CHECK(y_partials(job, st, C, n, cj12, ck12, nbf5, nalpha, nbeta, &ypart, &nparts));
     // H_mat = C^T (H C5) (src/utils.jl:17-18), elag = [n o H_mat + C^T Y | 0], E_elec
-    return elag_tail_f64(job, st, C, H, n, nbf5, ypart, false, nparts, (long long)nbf * nbf5, Hmat, elag, E);
+    return elag_tail_f64(job, st, C, H, n, nbf5, ypart, false, nparts, (long long)nbf * nbf5, Hmat, elag, E, true);
 }
 
 // The Lagrangian of a slice of the aux index (the job's b holds naux_r aux
@@ -448,7 +457,7 @@ int lagrange2_f64_noalloc(donof_job* job, cudaStream_t st, const double* C, cons
     {
         double* tv = W + (size_t)Kt * nbf5;
         w_diag_kernel<<<grid_for(wbuild::diag_units(nbf5, naux) * 256, 256, ctx->sm_count), 256, 0, st>>>(
-            bpq, n, cj12, nbf5, naux, nalpha, nbeta, tv); count_launch();
+            bpq, n, cj12, nbf5, naux, nalpha, nbeta, tv, nullptr); count_launch();
         build_w_kernel<<<grid_for(wbuild::tiles(nbf5, naux) * 256, 256, ctx->sm_count), 256, 0, st>>>(
             bpq, ck12, tv, nbf5, naux, W); count_launch();
         DONOF_CUDA(ctx, cudaGetLastError());

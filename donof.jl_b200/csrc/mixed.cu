@@ -596,7 +596,8 @@ __global__ void split_c_kernel(const double* __restrict__ C, int nbf, int nbf5, 
 // n32[q], cj32[q + 64 c] = cj12[q, c], ck32[q + 64 b] = ck12[b, q]
 __global__ void prep_coef_kernel(const double* __restrict__ n, const double* __restrict__ cj12,
                                  const double* __restrict__ ck12, int nbf5, float* __restrict__ n32,
-                                 float* __restrict__ cj32, float* __restrict__ ck32) {
+                                 float* __restrict__ cj32, float* __restrict__ ck32, unsigned* tail_words) {
+    zero_tail_state(tail_words);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 64 * 64; i += gridDim.x * blockDim.x) {
         const int r = i & 63, c = i >> 6;
         const bool in = r < nbf5 && c < nbf5;
@@ -857,7 +858,7 @@ int split_c_grouped(donof_ctx* ctx, cudaStream_t st, const MixedSplitJob* d_jobs
 
 int prep_coef(donof_ctx* ctx, cudaStream_t st, const double* n, const double* cj12, const double* ck12, int nbf5,
               float* n32, float* cj32, float* ck32) {
-    mx::prep_coef_kernel<<<16, 256, 0, st>>>(n, cj12, ck12, nbf5, n32, cj32, ck32); count_launch();
+    mx::prep_coef_kernel<<<16, 256, 0, st>>>(n, cj12, ck12, nbf5, n32, cj32, ck32, nullptr); count_launch();
     DONOF_CUDA(ctx, cudaGetLastError());
     return DONOF_OK;
 }
@@ -929,11 +930,14 @@ int lagrange2_mixed(donof_job* job, cudaStream_t st, const double* C, const doub
     const int nbf = job->nbf, grid = mixed_grid(job);
     MixedScratch S;
     DONOF_CHECK(mixed_prepare(job, st, C, nbf5, &S, grid));
-    mx::prep_coef_kernel<<<16, 256, 0, st>>>(n, cj12, ck12, nbf5, S.n32, S.cj32, S.ck32); count_launch();
+    unsigned* words = nullptr;
+    DONOF_CHECK(tail_state(job, nbf5, &words));
+    mx::prep_coef_kernel<<<16, 256, 0, st>>>(n, cj12, ck12, nbf5, S.n32, S.cj32, S.ck32, words); count_launch();
     DONOF_CUDA(ctx, cudaGetLastError());
     DONOF_CHECK(launch_mixed(job, st, nbf5, nalpha, nbeta, 3, S, nullptr, nullptr, grid));
     // Y (FP64) = sum over CTAs of the FP32 partials; H_mat, elag and E_elec in FP64
-    return elag_tail_f64(job, st, C, H, n, nbf5, S.ypart, true, grid, (long long)nbf * nbf5, Hmat, elag, E);
+    return elag_tail_f64(job, st, C, H, n, nbf5, S.ypart, true, grid, (long long)nbf * nbf5, Hmat, elag, E,
+                         true);
 }
 
 int jkh_mo_mixed(donof_job* job, cudaStream_t st, const double* C, const double* H, int nbf5, double* J, double* K,

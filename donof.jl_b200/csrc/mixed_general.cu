@@ -363,8 +363,9 @@ constexpr int WQ = 512;  // diagonal elements staged at a time
 
 __global__ void __launch_bounds__(256) mg_wdiag_kernel(const float* __restrict__ bpq, const float* __restrict__ n32,
                                                        const float* __restrict__ cj32, int nbf5, int naux, int nalpha,
-                                                       int nbeta, float* __restrict__ tv) {
+                                                       int nbeta, float* __restrict__ tv, unsigned* tail_words) {
     __shared__ __align__(16) float sd[WQ][WL];
+    zero_tail_state(tail_words);
     const long long n55 = (long long)nbf5 * nbf5;
     const int l0 = blockIdx.x * WL;
     for (int b0 = 0; b0 < nbf5; b0 += blockDim.x) {
@@ -624,11 +625,13 @@ int lagrange2_mixed_general(donof_job* job, cudaStream_t st, const double* C, co
     const int nbf = job->nbf, naux = job->naux;
     GenScratch S;
     DONOF_CHECK(gen_prepare(job, st, C, n, cj12, ck12, nbf5, true, &S));
+    unsigned* words = nullptr;
+    DONOF_CHECK(tail_state(job, nbf5, &words));
     DONOF_CHECK(gen_transforms(job, st, nbf5, S));
     {
         const int threads = nbf5 >= 256 ? 256 : (nbf5 + 31) / 32 * 32;
         mg::mg_wdiag_kernel<<<(naux + mg::WL - 1) / mg::WL, threads, 0, st>>>(S.bpq, S.n32, S.cj32, nbf5, naux,
-                                                                             nalpha, nbeta, S.tv); count_launch();
+                                                                             nalpha, nbeta, S.tv, words); count_launch();
         long long blocks = ((long long)nbf5 * naux + 7) / 8;
         if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
         mg::mg_w_kernel<<<(int)blocks, 256, 0, st>>>(S.bpq, S.ckT, S.tv, nbf5, S.ldq, naux, S.w_hi,
@@ -658,7 +661,8 @@ int lagrange2_mixed_general(donof_job* job, cudaStream_t st, const double* C, co
     P.lchunk = S.lchunk; P.nchunks = S.nchunks;
     P.out = S.ypart;
     DONOF_CHECK(launch_gemm(job, st, P, w_hi, w_lo, tm_hi, tm_lo));
-    return elag_tail_f64(job, st, C, H, n, nbf5, S.ypart, true, S.nchunks, (long long)nbf * nbf5, Hmat, elag, E);
+    return elag_tail_f64(job, st, C, H, n, nbf5, S.ypart, true, S.nchunks, (long long)nbf * nbf5, Hmat, elag, E,
+                         true);
 }
 
 int transforms_mixed_general(donof_job* job, cudaStream_t st, const double* C, int nbf5) {

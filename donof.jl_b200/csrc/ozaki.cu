@@ -897,7 +897,9 @@ __global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ D,
                                                    const double* __restrict__ cj12, int nbf5, int naux, int nalpha,
                                                    int nbeta, const double* __restrict__ RL,
                                                    const double* __restrict__ CN, const double* __restrict__ beta,
-                                                   double* __restrict__ tv, unsigned* __restrict__ wmax) {
+                                                   double* __restrict__ tv, unsigned* __restrict__ wmax,
+                                                   unsigned* tail_words) {
+    zero_tail_state(tail_words);
     __shared__ double sd[LB][DQ];
     __shared__ double part[8][LB][32];   // [warp][l][b]
     const int l0 = blockIdx.x * LB, b = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
@@ -1252,7 +1254,7 @@ int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const dou
 // W from job->bpq and Y = sum_l tmp_l W_l as FP64 partials (nbf x nbf5 each) in
 // job->part, after transforms_ozaki with the same coefficients.
 int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12, const double* ck12, int nbf5,
-            int nalpha, int nbeta, const double** ypart, int* nparts) {
+            int nalpha, int nbeta, const double** ypart, int* nparts, unsigned* tail_words) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux, ldq = ldq_of(nbf5), nch = chunks_of(nbf5, naux);
     const size_t wbytes = (size_t)oz::S * nbf5 * oz::KC * nch;
@@ -1264,7 +1266,8 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
     const double* bpq = job->bpq.as<double>();
     {
         const dim3 grid((naux + oz::LB - 1) / oz::LB, (nbf5 + 31) / 32);
-        oz::diag_kernel<<<grid, 256, 0, st>>>(bpq + (size_t)nbf5 * nbf5 * naux, n, cj12, nbf5, naux, nalpha, nbeta, P.RL, P.CN, P.beta, tv, P.wmax);
+        oz::diag_kernel<<<grid, 256, 0, st>>>(bpq + (size_t)nbf5 * nbf5 * naux, n, cj12, nbf5, naux, nalpha, nbeta,
+                                              P.RL, P.CN, P.beta, tv, P.wmax, tail_words);
         count_launch();
     }
     {

@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(dtile::THREADS) elag_tail_kernel(const TailArg
 }
 
 static_assert(sizeof(TailState) <= GROUP_STATE_BYTES, "tail state slot too small");
+static_assert(sizeof(TailState) == sizeof(unsigned) * TAIL_STATE_WORDS, "tail state words");
 
 // Grouped form: the tails of several jobs in one cooperative launch, job j on
 // CTAs [cta0, cta0 + ctas) with its own barrier state (as rotate_grouped_kernel).
@@ -259,14 +260,21 @@ int tail_grouped(donof_ctx* ctx, cudaStream_t st, const TailJob* jobs, int njobs
     return DONOF_OK;
 }
 
+int tail_state(donof_job* job, int nbf5, unsigned** words) {
+    DONOF_CHECK(job->small.ensure(job->ctx, 256 + sizeof(double) * 2 * (size_t)job->nbf * nbf5));
+    *words = job->small.as<unsigned>();
+    return DONOF_OK;
+}
+
 int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double* H, const double* n, int nbf5,
                   const void* part, bool part_f32, int nparts, long long pstride, double* Hmat, double* elag,
-                  double* E) {
+                  double* E, bool state_zeroed) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf;
     const size_t ny = (size_t)nbf * nbf5;
-    DONOF_CHECK(job->small.ensure(ctx, 256 + sizeof(double) * 2 * ny));
-    char* base = job->small.as<char>();
+    unsigned* words = nullptr;
+    DONOF_CHECK(tail_state(job, nbf5, &words));
+    char* base = reinterpret_cast<char*>(words);
     TailArgs a{};
     a.C = C; a.H = H; a.n = n;
     a.nbf = nbf; a.nbf5 = nbf5;
@@ -290,7 +298,7 @@ int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double
         return DONOF_ERR_CUDA;
     }
     const int grid = ctx_ctas(ctx);  // at most one CTA per SM (co-resident: the kernel has grid barriers)
-    DONOF_CUDA(ctx, cudaMemsetAsync(a.ts, 0, sizeof(TailState), st));
+    if (!state_zeroed) DONOF_CUDA(ctx, cudaMemsetAsync(a.ts, 0, sizeof(TailState), st));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(dtile::THREADS);
