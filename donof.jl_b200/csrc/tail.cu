@@ -297,7 +297,13 @@ int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double
         set_error(ctx, "elag_tail_kernel does not fit on an SM");
         return DONOF_ERR_CUDA;
     }
-    const int grid = ctx_ctas(ctx);  // at most one CTA per SM (co-resident: the kernel has grid barriers)
+    // At most one CTA per SM (co-resident: the kernel has a grid barrier), and no more than
+    // have a tile or a block of the reduction in stage 1 or a tile in stage 2 (tail at nbf =
+    // 24, nbf5 = 20: 7.4 us on 10 CTAs, 8.2 on 148).  A sum does not depend on the grid.
+    const int nt = (nbf + dtile::TM - 1) / dtile::TM * ((nbf5 + TL_TN - 1) / TL_TN);
+    const size_t stage1 = nt + (ny + 63) / 64, most = stage1 > 2 * (size_t)nt ? stage1 : 2 * (size_t)nt;
+    int grid = ctx_ctas(ctx);
+    if ((size_t)grid > most) grid = (int)most;
     if (!state_zeroed) DONOF_CUDA(ctx, cudaMemsetAsync(a.ts, 0, sizeof(TailState), st));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
