@@ -598,7 +598,7 @@ def batched_bench(d, torch, ctx, steps, warmup, method, sequential_arm=True, spe
                        f"nbf5 20k), FP64, {steps} orbital steps each",
            "ks": [k for k, _ in jobs], "unit": "job orbital-gradient steps/s",
            "grouped": {"value": nj * steps / tg, "ms_per_step": 1e3 * tg / steps, "launches_per_step": lg / steps,
-                       "path": "donof_batch_orbopt (grouped persistent GEMMs + grouped cooperative kernels, "
+                       "path": "donof_batch_orbopt (grouped GEMMs + grouped cooperative kernels, "
                                "one graph)"},
            "sequential": {"value": nj * steps / ts, "ms_per_round": 1e3 * ts / steps,
                           "path": "donof_orbopt_dev per job, one after the other"},
@@ -883,13 +883,14 @@ def main():
     peaks = load_peaks()
     if args.precision == "fp64" and bt.fp64_tc:
         ldn = (nbf + 15) // 16 * 16
-        byts = 7.0 * nbf * ldn * naux + 8.0 * nbf * nbf5 * naux
+        ldq = (nbf5 + 15) // 16 * 16
+        byts = 7.0 * nbf * ldn * naux + 7.0 * nbf * ldq * naux
         macs = 28.0 * nbf * nbf * nbf5 * naux
         roof = {"bound": "hbm", "achieved": byts / tr / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": byts / tr / 1e9 / peaks["hbm_gbs"], "traffic": traffic_from_profiles("t1_oz"),
-                "kernel": "ozaki_t1_kernel (T1 tmp_l = b_l C5 on tcgen05 kind::i8: 28 digit products, "
-                          "int32 TMEM accumulators, FP64 recombination)",
-                "algorithmic": f"int8 slices of b read once + tmp written = 7*nbf*ldn*naux + 8*nbf*nbf5*naux "
+                "kernel": "oz_kernel<T1_DIGITS> (T1 tmp_l = b_l C5 on tcgen05 kind::i8: 28 digit products, "
+                          "int32 TMEM accumulators, FP64 recombination, tmp as digit slices)",
+                "algorithmic": f"int8 slices of b read once + of tmp written = 7*nbf*ldn*naux + 7*nbf*ldq*naux "
                                f"= {byts:.4e} bytes per launch",
                 "int8_tops": 2.0 * macs / tr / 1e12, "fp64_equivalent_tflops": 2.0 * nbf * nbf * nbf5 * naux / tr / 1e12,
                 "ms": tr * 1e3,

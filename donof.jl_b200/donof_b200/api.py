@@ -147,9 +147,9 @@ class BTensor:
         self.precision = prec
 
     def set_fp64_tc(self, enable: bool = True) -> None:
-        """Run the FP64 form's first contraction (tmp_l = b_l C5) on the tensor
-        cores from int8 digit slices of b (made now, 7/8 of b's FP64 size), or
-        back on the FP64 GEMM (enable=False frees the slices)."""
+        """Run the FP64 form's contractions on the tensor cores from int8 digit
+        slices (b's made now, 7/8 of its FP64 size), or back on the FP64 GEMM
+        (enable=False frees the slices)."""
         self.ctx.check(self.ctx.lib.donof_job_set_fp64_tc(self.handle, 1 if enable else 0))
 
     @property

@@ -43,10 +43,10 @@ PRECISIONS = ("fp64", "mixed", "mixed_refined", "auto")
 AUTO_MIXED_MIN_WORK = 2.0e7
 
 
-# The FP64 form's first contraction runs on the tensor cores from int8 digit
-# slices of b (ozaki.cu) for jobs of at least this many basis functions: there
-# it is faster than the DMMA GEMM (nbf = 202: 450 against 746 us per call,
-# nbf = 256: 130 against 290 us); below, the contraction is a few microseconds
+# The FP64 form's contractions run on the tensor cores from int8 digit slices
+# of b (ozaki.cu) for jobs of at least this many basis functions: there they are
+# faster than the DMMA GEMM (the first one at nbf = 202: 273 against 746 us,
+# nbf = 256: 106 against 290 us); below, a contraction is a few microseconds
 # either way and the slices would only cost memory.
 FP64_TC_MIN_NBF = 128
 

@@ -112,7 +112,7 @@ end
 set_precision!(b::B200Tensor, precision::Integer) =
     check(ccall((:donof_job_set_precision, libdonof), Cint, (Ptr{Cvoid}, Cint), b.job, precision))
 
-"""FP64 form: run the first contraction (b_l C5) on the tensor cores from int8 digit
+"""FP64 form: run the contractions on the tensor cores from int8 digit
 slices of b (exact integer products, within ~1e-13 of the FP64 GEMM), or back on the
 FP64 GEMM with `enable = false`."""
 set_fp64_tc!(b::B200Tensor, enable::Bool=true) =
