@@ -41,8 +41,7 @@ cudaError_t launch_persistent(const GemmF64Args& p, cudaStream_t st) {
     long long grid = (long long)per_sm_cached.load(std::memory_order_acquire) * sm_cached.load(std::memory_order_acquire);
     if (grid > total) grid = total;
     if (grid < 1) grid = 1;
-    kern<<<(unsigned)grid, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p); count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(kern, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 template <int BM, int BN, int WM, int WN, bool AK, bool BKM, bool VEC>
@@ -64,8 +63,7 @@ cudaError_t launch_cfg(const GemmF64Args& p, cudaStream_t st, bool persistent) {
         attr_mask.fetch_or(bit, std::memory_order_acq_rel);
     }
     dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN, p.batch * p.splits);
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, st>>>(p); count_launch();
-    return cudaGetLastError();
+    return launch_overlapped(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, st, p);
 }
 
 template <int BM, int BN, int WM, int WN, bool AK, bool BKM>

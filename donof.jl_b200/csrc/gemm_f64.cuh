@@ -59,6 +59,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The start of a kernel that launch_overlapped starts early: nothing of the kernels before
+// it may be read or overwritten before this returns (they have completed, their writes
+// are visible).
+__device__ __forceinline__ void stream_order() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Before a CTA's last stores: once every CTA has come so far, the next kernel of the
+// stream may be brought onto the SMs.  (Said at the start instead, its waiting CTAs take
+// the room of this kernel's: the Lagrangian at nbf = 91 137 against 117 us, and no gain
+// at nbf = 24: 22 us either way, 28 with ordinary launches.)
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src, bool valid) {
     const uint32_t d = smem_u32(dst);
@@ -322,6 +332,7 @@ template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK,
 __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N)
 gemm_f64_kernel(const GemmF64Args p) {
     extern __shared__ __align__(16) double smem[];
+    gemm_detail::stream_order();
     using Tile = GemmTileF64<BM, BN, BK, WARPS_M, WARPS_N, STAGES, AK, BKM, VEC>;
     Tile T;
     T.init(p, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -330,6 +341,7 @@ gemm_f64_kernel(const GemmF64Args p) {
     T.prologue(smem);
     T.mainloop(smem, acc);
     gemm_detail::cp_async_wait<0>();
+    gemm_detail::let_next_start();
     T.epilogue(acc);
 }
 
@@ -350,6 +362,7 @@ template <int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, bool AK,
 __global__ void __launch_bounds__(32 * WARPS_M * WARPS_N, (persistent_min_ctas<BM, BN, WARPS_M, WARPS_N>()))
 gemm_f64_persistent_kernel(const GemmF64Args p) {
     extern __shared__ __align__(16) double smem[];
+    gemm_detail::stream_order();
     using Tile = GemmTileF64<BM, BN, BK, WARPS_M, WARPS_N, STAGES, AK, BKM, VEC>;
     const int gx = (p.M + BM - 1) / BM, gy = (p.N + BN - 1) / BN;
     const int total = gx * gy * p.batch * p.splits;
@@ -370,6 +383,7 @@ gemm_f64_persistent_kernel(const GemmF64Args p) {
             __syncthreads();  // every warp is done with the stages the prologue overwrites
             nxt.prologue(smem);
         }
+        if (!more) gemm_detail::let_next_start();
         cur.epilogue(acc);
         if (!more) break;
         cur = nxt;

@@ -73,6 +73,30 @@ int gemm_f64_partials_splits(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, boo
 // Fused FP64 tail of the Lagrangian (tail.cu): Y = sum of nparts partials
 // (FP32 or FP64, part[g * pstride + m + nbf * b]), HC = H C5, H_mat = C^T HC,
 // elag = [n o H_mat + C^T Y | 0] and E_elec (when E != nullptr).
+// Launches a kernel that starts with gemm_detail::stream_order() so that its CTAs are
+// brought in while the kernel before it ends (programmatic dependent launch); in a
+// captured graph an ordinary launch.
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const bool asked = cudaStreamIsCapturing(st, &cs) == cudaSuccess;
+    if (!asked) cudaGetLastError();
+    const bool plain = !asked || cs != cudaStreamCaptureStatusNone;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = plain ? 0 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    count_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // The tail's barrier state: tail_state returns its TAIL_STATE_WORDS words (in job->small,
 // sized for the tail), which a kernel that runs earlier in the call zeroes with
 // zero_tail_state; elag_tail_f64 is then told so and needs no memset of its own.

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(256, 4) build_w_fused_kernel(const double* __r
                                                             const double* __restrict__ ck12, int nbf5, int naux,
                                                             int nalpha, int nbeta, double* __restrict__ W,
                                                             unsigned* tail_words) {
+    gemm_detail::stream_order();
     zero_tail_state(tail_words);
     __shared__ double tb[wbuild::LT][32][33];
     __shared__ double sd[wbuild::LT * FUSED_W_MAX];
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(256, 4) build_w_fused_kernel(const double* __r
                 tb[k][ty + 8 * r][tx] = w;  // [l - l0][q - q0][b - b0]
             }
         }
+        if (t + gridDim.x >= tiles) gemm_detail::let_next_start();
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < wbuild::LT; ++k) {
@@ -187,9 +189,8 @@ int build_w(donof_ctx* ctx, cudaStream_t st, const double* bpq, const double* n,
     long long blocks = wbuild::tiles(nbf5, naux);
     if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
     if (nbf5 <= FUSED_W_MAX) {
-        build_w_fused_kernel<<<(int)blocks, 256, 0, st>>>(bpq, n, cj12, ck12, nbf5, naux, nalpha, nbeta, W,
-                                                        tail_words);
-        count_launch();
+        DONOF_CUDA(ctx, launch_overlapped(build_w_fused_kernel, dim3((unsigned)blocks), 256, 0, st, bpq, n, cj12, ck12,
+                                          nbf5, naux, nalpha, nbeta, W, tail_words));
     } else {
         double* tv = W + (size_t)nbf5 * naux * nbf5;  // n'_b d_b^l + t_b^l (Kt values)
         long long dblocks = wbuild::diag_units(nbf5, naux);
