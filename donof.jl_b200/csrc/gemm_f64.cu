@@ -342,7 +342,7 @@ const int kTileBM[kNT] = {128, 64, 32, 64}, kTileBN[kNT] = {64, 64, 32, 64};
 // they lose (T1 at 96 x 96 x 96, 464 products: 35 and 31 us against 33; 192 x 160 x 192,
 // 928 products: 387 and 371 against 353); with less they gain (91 x 66 x 91, 437
 // products: 29 and 31 us against 35; 96 x 80 x 96, 464 products: 31 us against 33).
-int narrow_tiles(bool b_kmajor, int M, int N, GemmTile (&tiles)[2], int (&bm)[2], int (&bn)[2]) {
+int narrow_tiles(bool b_kmajor, int M, int N, GemmTile* tiles, int* bm, int* bn) {
     if (!b_kmajor) return 0;
     auto padded = [&](int tm, int tn) { return (long long)((M + tm - 1) / tm * tm) * ((N + tn - 1) / tn * tn); };
     int n = 0;
@@ -397,33 +397,41 @@ int partials_choice(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, bool b_kmajo
     p.M = M; p.N = N; p.K = K;
     p.A = A; p.lda = lda; p.B = B; p.ldb = ldb;
     p.alpha = 1.0; p.beta = 0.0; p.batch = 1; p.splits = 1; p.kchunk = K;
-    // candidates: each tile shape with about one and about two CTAs per SM, the small
-    // tiles, of which six to eight fit, with up to four
+    // candidates: each tile shape with about one and about two CTAs per SM, and the small
+    // tiles, of which six to eight fit, with the split counts of the others too (a count
+    // of its own would make another sum; Y at nbf = 91, nbf5 = 66, naux = 437 in 28 us on
+    // 48 x 24 tiles, 33 with two CTAs per SM of 32 x 32)
     std::vector<TuneVal> cands;
     {
         int sp = 1;
         const GemmTile h = pick_tile(ctx, M, N, K, true, &sp);
         cands.push_back(TuneVal{h, sp});
         const int max_splits = K / 64 > 1 ? K / 64 : 1;
-        auto add = [&](GemmTile tile, int bm, int bn) {
-            const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-            const int most = bm * bn <= 32 * 40 ? 4 : 2;
-            for (int f = 1; f <= most; ++f) {
+        auto tiles_of = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+        auto add = [&](GemmTile tile, int splits) {
+            for (const TuneVal& c : cands)
+                if (c.tile == tile && c.splits == splits) return;
+            cands.push_back(TuneVal{tile, splits});
+        };
+        for (int t = 0; t < kNT; ++t)
+            for (int f = 1; f <= 2; ++f) {
+                const long long tiles = tiles_of(kTileBM[t], kTileBN[t]);
                 long long s = (f * (long long)ctx->sm_count + tiles - 1) / tiles;
                 if (s > max_splits) s = max_splits;
                 if (s < 1) s = 1;
-                bool dup = false;
-                for (const TuneVal& c : cands) dup = dup || (c.tile == tile && c.splits == (int)s);
-                if (!dup) cands.push_back(TuneVal{tile, (int)s});
+                add(kTiles[t], (int)s);
             }
-        };
-        for (int t = 0; t < kNT; ++t) add(kTiles[t], kTileBM[t], kTileBN[t]);
         const size_t nplain = cands.size();
         for (size_t c = 0; c < nplain; ++c) cands.push_back(TuneVal{cands[c].tile, cands[c].splits, true});
-        GemmTile narrow[2];
-        int bm[2], bn[2];
-        const int nn = narrow_tiles(b_kmajor, M, N, narrow, bm, bn);
-        for (int t = 0; t < nn; ++t) add(narrow[t], bm[t], bn[t]);
+        GemmTile narrow[3];
+        int bm[3], bn[3];
+        int nn = narrow_tiles(b_kmajor, M, N, narrow, bm, bn);
+        narrow[nn] = GemmTile::Tiny;
+        bm[nn] = bn[nn] = 32;
+        ++nn;
+        for (int t = 0; t < nn; ++t)
+            for (size_t c = 0; c < nplain; ++c)
+                if (tiles_of(bm[t], bn[t]) * cands[c].splits <= 5LL * ctx->sm_count) add(narrow[t], cands[c].splits);
     }
     auto config = [&](const TuneVal& c, GemmF64Args* q, int* ns) {
         *q = p;
