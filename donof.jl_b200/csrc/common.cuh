@@ -136,6 +136,7 @@ struct donof_job {
     void* oz_b = nullptr;
     donof::DevBuf oz_c;
     unsigned oz_gen = 0;
+    bool oz_t1_only = false;  // b's rows differ too much in size for tmp's and W's digits
     // per-call scratch, sized for the largest nbf5 seen
     donof::DevBuf tmp, bpq, W, part, small;
     // device-resident orbital-optimiser state

@@ -211,18 +211,20 @@ int grid_for(long long total, int threads, int sm) {
 
 }  // namespace
 
-// T1 + T2 into the job scratch: tmp (nbf x nbf5 x naux; digit slices of it with
-// b's digit slices on the device, see ozaki.cu) and bpq (nbf5^2 x naux).
+// T1 + T2 into the job scratch: tmp (nbf x nbf5 x naux; digit slices of it where the
+// contractions run from digits, see ozaki.cu) and bpq (nbf5^2 x naux).
 int transforms_f64(donof_job* job, cudaStream_t st, const double* C, int nbf5) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
-    if (job->oz_b) return transforms_ozaki(job, st, C, nullptr, nullptr, nullptr, nbf5);
+    if (ozaki_products(job)) return transforms_ozaki(job, st, C, nullptr, nullptr, nullptr, nbf5);
     DONOF_CHECK(job->tmp.ensure(ctx, sizeof(double) * (size_t)nbf * nbf5 * naux));
     DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * nbf5 * naux));
     double* tmp = job->tmp.as<double>();
     double* bpq = job->bpq.as<double>();
     // T1: tmp_l(m,q) = sum_n b[m,n,l] C[n,q]; A(i=m,k=n) = b[m + nbf*n] (M-contiguous).
-    {
+    if (job->oz_b) {
+        DONOF_CHECK(t1_ozaki(job, st, C, nbf5, tmp));
+    } else {
         GemmF64Args p{};
         p.M = nbf; p.N = nbf5; p.K = nbf;
         p.A = job->b; p.lda = nbf; p.strideA = (long long)nbf * nbf;
@@ -257,7 +259,7 @@ int y_partials(donof_job* job, cudaStream_t st, const double* C, const double* n
     const int nbf = job->nbf, naux = job->naux;
     unsigned* words = nullptr;
     DONOF_CHECK(tail_state(job, nbf5, &words));
-    if (job->oz_b) {
+    if (ozaki_products(job)) {
         DONOF_CHECK(transforms_ozaki(job, st, C, n, cj12, ck12, nbf5));
         return y_ozaki(job, st, n, cj12, ck12, nbf5, nalpha, nbeta, ypart, nparts, words);
     }

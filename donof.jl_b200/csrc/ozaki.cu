@@ -22,17 +22,30 @@
 //         written by T1's epilogue with no pass for a maximum; the bound is 2-3
 //         bits above the largest value
 //   W     balanced digits of RL[l] CN[q] W_l[q, b], one scale per b (beta_b times the
-//         largest |RL CN b_pq| and |RL CN t|, found by T2's epilogue and the
-//         diagonal kernel), so that tmp's scales drop out of Y's sum over (q, l)
+//         largest |RL CN b_pq[b, q]| of that b, and the largest |RL CN t_b|, found by
+//         T2's epilogue and the diagonal kernel), so that tmp's scales drop out of Y's
+//         sum over (q, l)
 // A product keeps the digit pairs with i + j < NG, NG = 7 in T1 and 8 in T2 and Y:
 // exact s8 x s8 -> s32 sums (tcgen05.mma kind::i8) in NG TMEM accumulators (one per
 // i + j, 64 columns each), combined in FP64 by the epilogue (exact int32 -> double,
 // Horner in 2^-7 or 2^-8).  |sum| <= 7 * 2^14 * K < 2^31 for K <= 18688; Y's K range is
 // cut accordingly.
-// T1 is within 1e-13 of the FP64 product, T2 and Y are as near to theirs as an FP64
-// GEMM (error of b_pq 1.4e-16 of the norm, of Y 2.1e-16, the GEMM's 3.3e-16 and
-// 9.7e-16, nbf = 96, random b; NG = 7 left 1.6e-15 in Y).  The optimisers divide by
-// gradient elements, so noise of 1e-14 in T2 and Y showed as 1e-8 in the orbitals.
+// T1 is within 1e-13 of the FP64 product, row by row of b_l.  T2 and Y are, by the norm,
+// as near to theirs as an FP64 GEMM (error of b_pq 1.4e-16 of the norm, of Y 2.1e-16, the
+// GEMM's 3.3e-16 and 9.7e-16, nbf = 96, random b; NG = 7 left 1.6e-15 in Y).  The
+// optimisers divide by gradient elements, so noise of 1e-14 in T2 and Y showed as 1e-8 in
+// the orbitals.
+//
+// What is held in fixed point is relative to a bound of many elements: tmp to the largest
+// row of b_l, column b of W to its largest term.  Elements far below lose bits that FP64
+// would keep (three water molecules, orbitals of the core Hamiltonian: the median element
+// of b_pq is off by 2.2e-12 of itself instead of 2.0e-12; J, K, Y and elag, sums over l,
+// are not further off).  A row m of Y is as good as T1's noise (2^-44) allows while its
+// largest row norm over l is within 2^6 of the largest of all rows: 2^-57 2^6 from tmp's
+// digits, and as much again squared from W's where the orbitals are the basis functions
+// themselves.  Molecules lie within that (water: 5).  A job whose rows spread further
+// (ROW_SPREAD) keeps T1 from digits and takes T2 and Y as FP64 GEMMs: on rows 1e-9 and
+// 1e6 times the others the digit products left nothing of the small rows.
 //
 // One persistent kernel, oz_kernel<MODE>, with TMEM accumulators of 64 columns each
 // for a 128 x 64 output tile: warp 16 streams A's slices (16 KB TMA boxes, no
@@ -79,13 +92,14 @@ namespace oz {
 constexpr int S = 7;                        // digits of every operand
 constexpr int NG_MAX = 8;                   // accumulators: digit pairs with i + j < NG
 constexpr double F = 0.498;                 // largest |x| / scale: every balanced digit fits [-128, 127]
+constexpr double ROW_SPREAD = 64.0;         // largest ratio of b's row norms that T2 and Y take as digits
 constexpr int EPI_WARPS = 16;               // four per TMEM lane quarter, 16 columns each (8 of 32: T1 148 against 113 us at nbf5 = 64)
 constexpr int PRODUCER = EPI_WARPS;         // TMA producer
 constexpr int ISSUER = EPI_WARPS + 1;       // TMEM allocator + MMA issuer
 constexpr int NTHREADS = 32 * (EPI_WARPS + 2);
 // 18 warps put 5 on one SM sub-partition of 16384 registers: at most 96 per thread
 constexpr int BOUND_THREADS = 640;
-constexpr int KC = 128;                     // K per stage: one 128-byte swizzle row of int8
+constexpr int KC = 128;                     // K per stage: eight 16-byte groups of int8
 constexpr int MT = 128;                     // rows per tile (MMA M)
 constexpr int QT = 64;                      // columns per tile (MMA N per B slice)
 constexpr int A_BYTES = MT * KC;            // 16 KB: one slice of A over (row tile, K chunk)
@@ -139,7 +153,7 @@ struct Params {
     const double* sb1;         // per q: 2^(eb - 14), of C5's truncated digits
     const double* sb2;         // per q: s 2^-16, of its balanced digits
     const double* beta;        // per b (Y)
-    unsigned* wmax;            // [0] of |RL CN b_pq|, [1] of |RL CN t| / beta: high words of the largest value
+    unsigned *wm, *wt;         // per b: high words of the largest |RL CN b_pq[b, q]| (T2; null: not wanted) and |RL CN t_b|
     int8_t* t8;                // tmp's slices (see the layout above t8_at)
     double* out;               // FP64 output
     double* diag;              // T2: b_qq^l at q + nbf5 l
@@ -211,14 +225,11 @@ __device__ __forceinline__ double value_above(unsigned hi) {
     return __hiloint2double((int)(hi < 0x7ff00000u ? hi + 1u : 0x7ff80000u), 0);
 }
 
-// The scale of W's digits over F: beta_b M with M an upper bound of the
-// largest |RL CN W| / beta (NaN when a term was not finite); 0 when W's row is zero.
-__device__ __forceinline__ double w_scale(double beta, const unsigned* wmax) {
-    double M = (value_above(wmax[0]) + value_above(wmax[1])) * (1.0 + 0x1p-40);
-    if (M < 1e-280) M = 1e-280;
-    double s = beta * M;
-    if (s < 1e-290) s = 0.0;
-    return s;
+// The scale over F of the digits of W's column b: an upper bound of its largest
+// |RL CN W| (NaN when a term was not finite); 0 when the column is zero.
+__device__ __forceinline__ double w_scale(double beta, unsigned wm, unsigned wt) {
+    const double s = (beta * value_above(wm) + value_above(wt)) * (1.0 + 0x1p-40);
+    return s < 1e-290 ? 0.0 : s;
 }
 
 // The work of one CTA: unit u = (row tile, column tile, K range).
@@ -578,7 +589,11 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
         __syncwarp();
         if (lane == 0)
             for (int g = 0; g < NG; ++g) mbar_arrive(bar(GFREE + g));
-        unsigned top = 0;  // T2: largest high word of |RL CN b_pq| of this thread
+        unsigned top = 0;  // T2: largest high word of |RL CN b_pq| in column `group NC + lane` of the tile
+        auto keep_top = [&](int q) {  // (lanes from NC on hold 0)
+            if (lane < NC && q + lane < P.nbf5) atomicMax(P.wm + q + lane, top);
+            top = 0;
+        };
         for (int u = 0; u < my_units; ++u) {
             const Unit w = unit_of<MODE, resident>(P, u);
             const int R = w.row * MT + quarter * 32 + lane;
@@ -652,9 +667,16 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                     if (in && q0 + k < P.nbf5) dst[(size_t)P.nbf * (q0 + k)] = v[k] * rs * P.sb1[q0 + k];
             } else if (MODE == T2) {
 #pragma unroll
-                for (int k = 0; k < NC; ++k) {
+                for (int k = 0; k < NC; ++k)
                     v[k] = v[k] * rs * P.sb2[q0 + k];  // b_pq (columns at and beyond nbf5: sb2 = 0)
-                    if (in) top = max(top, (unsigned)__double2hiint(v[k] * rs) & 0x7fffffffu);
+                if (P.wm != nullptr) {
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) {
+                        const unsigned h = __reduce_max_sync(
+                            0xffffffffu, in ? (unsigned)__double2hiint(v[k] * rs) & 0x7fffffffu : 0u);
+                        if (lane == k) top = max(top, h);
+                    }
+                    if (!resident || u == my_units - 1) keep_top(q0);
                 }
                 if (in && x >= q0 && x < q0 + NC) {
                     double t = 0.0;
@@ -679,12 +701,8 @@ oz_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
 #pragma unroll
                 for (int k = 0; k < NC; ++k)
                     if (in && q0 + k < P.nbf5)
-                        dst[(size_t)P.nbf * (q0 + k)] = v[k] * (w_scale(P.beta[q0 + k], P.wmax) * (0x1p-16 / F));
+                        dst[(size_t)P.nbf * (q0 + k)] = v[k] * (w_scale(P.beta[q0 + k], P.wm[q0 + k], P.wt[q0 + k]) * (0x1p-16 / F));
             }
-        }
-        if (MODE == T2) {
-            for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-            if (lane == 0) atomicMax(P.wmax, top);
         }
     }
 
@@ -719,10 +737,10 @@ __device__ __forceinline__ unsigned long long truncated7(double y) {
 __device__ __forceinline__ double digit_scale(double mx) { return fmax(mx, 1e-280) / F; }
 
 // Per row (m, l) of b: sa = 2^e with max_n |b| < 2^e (1 for a zero row), and the row
-// norm's maximum over m into rn[l] (bits of a non-negative double).  One thread per
-// (m, l), coalesced over m.
+// norm's maxima over m into rn[l] and over l into rm[m] (bits of a non-negative double).
+// One thread per (m, l), coalesced over m.
 __global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long long naux, double* __restrict__ sa,
-                                 unsigned long long* __restrict__ rn) {
+                                 unsigned long long* __restrict__ rn, unsigned long long* __restrict__ rm) {
     const long long total = (long long)nbf * naux;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -748,6 +766,28 @@ __global__ void row_scale_kernel(const double* __restrict__ b, int nbf, long lon
         if (mx > 0.0) frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1)
         sa[i] = isnan(norm) || isinf(mx) ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, e);
         atomicMax(rn + l, (unsigned long long)__double_as_longlong(norm));
+        atomicMax(rm + m, (unsigned long long)__double_as_longlong(norm));
+    }
+}
+
+// The largest of rm[0 .. nbf) and the smallest that is not zero (infinity if all are), by
+// one warp.
+__global__ void row_spread_kernel(const double* __restrict__ rm, int nbf, double* __restrict__ out) {
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    double hi = 0.0, lo = inf;
+#pragma unroll 4
+    for (int m = threadIdx.x; m < nbf; m += 32) {
+        const double x = rm[m];
+        hi = fmax(hi, x);
+        lo = fmin(lo, x > 0.0 ? x : inf);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+    if (threadIdx.x == 0) {
+        out[0] = hi;
+        out[1] = lo;
     }
 }
 
@@ -806,7 +846,7 @@ struct PrepArgs {
     int nbf, nbf5, nkc;             // grid: the columns rounded up to whole tiles
     double *sb1, *sb2, *CN, *cb, *beta;
     int8_t *c1, *c2;                // c8 of T1 and of T2, n padded to whole chunks with zeros
-    unsigned* wmax;
+    unsigned *wm, *wt;              // zeroed
 };
 
 // One block per column q of C5 (and per padding column): both sets of digit slices, the
@@ -815,7 +855,7 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
     __shared__ double red[3][4];
     __shared__ double bc[3];
     const int q = blockIdx.x, tid = threadIdx.x;
-    if (q == 0 && tid < 2) a.wmax[tid] = 0;
+    if (tid == 0) a.wm[q] = a.wt[q] = 0;
     if (q >= a.nbf5) {
         if (tid == 0) a.sb1[q] = a.sb2[q] = a.CN[q] = a.cb[q] = a.beta[q] = 0.0;
         return;
@@ -886,7 +926,7 @@ __global__ void __launch_bounds__(128) prep_kernel(const PrepArgs a) {
 
 // ---------------------------------------------------------------- W
 // tv[b + nbf5 l] = n'_b d_b^l + sum_q cj12[b, q] d_q^l with d_q^l = b_pq^l[q, q]
-// (lagrange.cu), and the largest |RL CN tv| / beta.  A block takes 32 b of LB aux
+// (lagrange.cu), and the largest |RL CN tv| per b.  A block takes 32 b of LB aux
 // indices: the diagonals (D, written by T2) staged in shared memory a panel of DQ at a time, each of
 // its eight warps on an eighth of the panel's q (one cj12 element, read along b,
 // serves LB products), the eight partial sums added in a fixed order.
@@ -896,12 +936,12 @@ constexpr int DQ = 256;
 __global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ D, const double* __restrict__ n,
                                                    const double* __restrict__ cj12, int nbf5, int naux, int nalpha,
                                                    int nbeta, const double* __restrict__ RL,
-                                                   const double* __restrict__ CN, const double* __restrict__ beta,
-                                                   double* __restrict__ tv, unsigned* __restrict__ wmax,
-                                                   unsigned* tail_words) {
+                                                   const double* __restrict__ CN, double* __restrict__ tv,
+                                                   unsigned* __restrict__ wt, unsigned* tail_words) {
     zero_tail_state(tail_words);
     __shared__ double sd[LB][DQ];
     __shared__ double part[8][LB][32];   // [warp][l][b]
+    __shared__ unsigned tops[LB][32];    // [l][b]
     const int l0 = blockIdx.x * LB, b = blockIdx.y * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
     double s[LB];
 #pragma unroll
@@ -933,11 +973,14 @@ __global__ void __launch_bounds__(256) diag_kernel(const double* __restrict__ D,
         const bool dj = (nbeta > 0) && (b < nbeta || b >= nalpha);
         if (dj) t = fma(n[b], D[(size_t)nbf5 * l + b], t);
         tv[b + (long long)nbf5 * l] = t;
-        const double be = beta[b];
-        top = (unsigned)__double2hiint(RL[l] * t * (be == 0.0 ? 0.0 : CN[b] / be)) & 0x7fffffffu;
+        top = (unsigned)__double2hiint(RL[l] * t * CN[b]) & 0x7fffffffu;
     }
-    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(wmax + 1, top);
+    tops[warp][threadIdx.x & 31] = top;
+    __syncthreads();
+    if (warp != 0 || b >= nbf5) return;
+#pragma unroll
+    for (int k = 1; k < LB; ++k) top = max(top, tops[k][threadIdx.x]);
+    atomicMax(wt + b, top);
 }
 static_assert(LB == 8, "one warp per aux index of a block");
 
@@ -950,7 +993,8 @@ __global__ void __launch_bounds__(256) w_digits_kernel(const double* __restrict_
                                                        const double* __restrict__ tv, int nbf5, int naux, int ldq,
                                                        int nch, const double* __restrict__ RL,
                                                        const double* __restrict__ CN, const double* __restrict__ beta,
-                                                       const unsigned* __restrict__ wmax, int8_t* __restrict__ W8) {
+                                                       const unsigned* __restrict__ wm,
+                                                       const unsigned* __restrict__ wt, int8_t* __restrict__ W8) {
     const int nbp = (nbf5 + 31) / 32 * 32;
     const long long total = (long long)nbp * nch * 8, n55 = (long long)nbf5 * nbf5;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -964,7 +1008,7 @@ __global__ void __launch_bounds__(256) w_digits_kernel(const double* __restrict_
         double v[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] = in && q0 + k < nbf5 ? B[(long long)nbf5 * (q0 + k)] : 0.0;
-        const double sc = w_scale(beta[b], wmax);
+        const double sc = w_scale(beta[b], wm[b], wt[b]);
         const double f = (sc == 0.0 || !in) ? 0.0 : RL[l] * (F * 0x1p56 / sc);
         const double td = (in && b >= q0 && b < q0 + 16) ? tv[b + (long long)nbf5 * l] : 0.0;
         unsigned wd[4][S];
@@ -997,24 +1041,26 @@ namespace {
 
 int ldn_of(int nbf) { return (nbf + 15) / 16 * 16; }  // 16-byte row pitch (TMA stride rule)
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-// one slice of b (whole 128-row tiles); the job's buffer holds the S slices, sa, RL and RLi
+// one slice of b (whole 128-row tiles); the job's buffer holds the S slices, sa, RL, RLi
+// and the spread of the row norms (two doubles)
 size_t slice_bytes(int nbf, int naux) { return ((size_t)naux * nbf + oz::MT - 1) / oz::MT * oz::MT * ldn_of(nbf); }
 
 struct JobLayout {
-    size_t sa, rl, bytes;
+    size_t sa, rl, spread, bytes;
 };
 JobLayout job_layout(int nbf, int naux) {
     JobLayout o;
     o.sa = align256(oz::S * slice_bytes(nbf, naux));
     o.rl = o.sa + align256(sizeof(double) * (size_t)nbf * naux);
-    o.bytes = o.rl + sizeof(double) * 2 * (size_t)naux;
+    o.spread = o.rl + sizeof(double) * 2 * (size_t)naux;
+    o.bytes = o.spread + sizeof(double) * 2;
     return o;
 }
 
 // C5's slices and the per-column arrays of a call, in job->oz_c
 struct CallLayout {
     int nq;
-    size_t c2, sb1, sb2, cn, cb, beta, wmax, bytes;
+    size_t c2, sb1, sb2, cn, cb, beta, wm, wt, bytes;
 };
 CallLayout call_layout(int nbf, int nbf5) {
     CallLayout o;
@@ -1026,8 +1072,9 @@ CallLayout call_layout(int nbf, int nbf5) {
     o.cn = o.sb2 + col;
     o.cb = o.cn + col;
     o.beta = o.cb + col;
-    o.wmax = o.beta + col;
-    o.bytes = o.wmax + 256;
+    o.wm = o.beta + col;
+    o.wt = o.wm + sizeof(unsigned) * (size_t)o.nq;
+    o.bytes = o.wm + col;
     return o;
 }
 
@@ -1077,7 +1124,8 @@ oz::Params base_params(donof_job* job, int nbf5) {
     P.CN = reinterpret_cast<double*>(cb + cl.cn);
     P.cb = reinterpret_cast<double*>(cb + cl.cb);
     P.beta = reinterpret_cast<double*>(cb + cl.beta);
-    P.wmax = reinterpret_cast<unsigned*>(cb + cl.wmax);
+    P.wm = reinterpret_cast<unsigned*>(cb + cl.wm);
+    P.wt = reinterpret_cast<unsigned*>(cb + cl.wt);
     P.fail = ctx->fail_dev ? ctx->fail_dev + FAIL_MBAR : nullptr;
     P.wait = sm100::wait_budget(ctx->wait_limit);
     return P;
@@ -1138,7 +1186,7 @@ int prep(donof_job* job, cudaStream_t st, const double* C, const double* n, cons
     a.sb1 = const_cast<double*>(P.sb1); a.sb2 = const_cast<double*>(P.sb2);
     a.CN = const_cast<double*>(P.CN); a.cb = const_cast<double*>(P.cb);
     a.beta = const_cast<double*>(P.beta);
-    a.c1 = job->oz_c.as<int8_t>(); a.c2 = a.c1 + cl.c2; a.wmax = P.wmax;
+    a.c1 = job->oz_c.as<int8_t>(); a.c2 = a.c1 + cl.c2; a.wm = P.wm; a.wt = P.wt;
     oz::prep_kernel<<<cl.nq, 128, 0, st>>>(a); count_launch();
     DONOF_CUDA(ctx, cudaGetLastError());
     return DONOF_OK;
@@ -1173,6 +1221,8 @@ int t1(donof_job* job, cudaStream_t st, int nbf5, double* out) {
 
 }  // namespace
 
+bool ozaki_products(const donof_job* job) { return job->oz_b && !job->oz_t1_only; }
+
 bool ozaki_shape_ok(int nbf) { return nbf >= 1 && nbf <= 16384; }
 
 size_t ozaki_bytes(int nbf, int naux) { return job_layout(nbf, naux).bytes; }
@@ -1193,17 +1243,23 @@ int ozaki_build(donof_job* job) {
     double* sa = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.sa);
     double* RL = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.rl);
     double* rn = RL + naux;
+    double* rm = static_cast<double*>(buf);  // row norms over l, until the slices take their place
+    double *spread = reinterpret_cast<double*>(static_cast<char*>(buf) + jl.spread), norms[2] = {0.0, 0.0};
     cudaStream_t st = ctx->stream;
     cudaError_t e = cudaMemsetAsync(rn, 0, sizeof(double) * (size_t)naux, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(rm, 0, sizeof(double) * (size_t)nbf, st);
     if (e == cudaSuccess) {
         oz::row_scale_kernel<<<8 * ctx->sm_count, 256, 0, st>>>(job->b, nbf, (long long)naux, sa,
-                                                               reinterpret_cast<unsigned long long*>(rn));
+                                                               reinterpret_cast<unsigned long long*>(rn),
+                                                               reinterpret_cast<unsigned long long*>(rm));
         count_launch();
+        oz::row_spread_kernel<<<1, 32, 0, st>>>(rm, nbf, spread); count_launch();
         oz::split_b_kernel<<<16 * ctx->sm_count, 256, 0, st>>>(job->b, sa, nbf, ldn_of(nbf), (long long)naux, slices);
         count_launch();
         oz::row_finish_kernel<<<(naux + 255) / 256, 256, 0, st>>>((long long)naux, RL, rn); count_launch();
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(norms, spread, sizeof(norms), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         dev_free(ctx, buf);
@@ -1211,6 +1267,7 @@ int ozaki_build(donof_job* job) {
         return DONOF_ERR_CUDA;
     }
     job->oz_b = buf;
+    job->oz_t1_only = norms[0] > oz::ROW_SPREAD * norms[1];
     ++job->oz_gen;
     return DONOF_OK;
 }
@@ -1248,6 +1305,7 @@ int transforms_ozaki(donof_job* job, cudaStream_t st, const double* C, const dou
     const int grid = shape_c5(ctx, P, (long long)P.ldq * naux);
     P.out = job->bpq.as<double>();
     P.diag = P.out + (size_t)nbf5 * nbf5 * naux;
+    if (n == nullptr) P.wm = nullptr;
     return launch_oz<oz::T2>(ctx, st, ma, mb, P, grid);
 }
 
@@ -1267,15 +1325,15 @@ int y_ozaki(donof_job* job, cudaStream_t st, const double* n, const double* cj12
     {
         const dim3 grid((naux + oz::LB - 1) / oz::LB, (nbf5 + 31) / 32);
         oz::diag_kernel<<<grid, 256, 0, st>>>(bpq + (size_t)nbf5 * nbf5 * naux, n, cj12, nbf5, naux, nalpha, nbeta,
-                                              P.RL, P.CN, P.beta, tv, P.wmax, tail_words);
+                                              P.RL, P.CN, tv, P.wt, tail_words);
         count_launch();
     }
     {
         const long long items = (long long)((nbf5 + 31) / 32 * 32) * nch * 8;
         long long blocks = (items + 255) / 256;
         if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
-        oz::w_digits_kernel<<<(int)blocks, 256, 0, st>>>(bpq, ck12, tv, nbf5, naux, ldq, nch, P.RL, P.CN, P.beta, P.wmax,
-                                                       w8);
+        oz::w_digits_kernel<<<(int)blocks, 256, 0, st>>>(bpq, ck12, tv, nbf5, naux, ldq, nch, P.RL, P.CN, P.beta, P.wm,
+                                                       P.wt, w8);
         count_launch();
     }
     DONOF_CUDA(ctx, cudaGetLastError());
