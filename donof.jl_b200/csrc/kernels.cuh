@@ -128,12 +128,13 @@ int iaux_f64(donof_ctx* ctx, cudaStream_t st, const double* G_host, const double
 // The FP64 form's contractions on the tensor cores from int8 digit slices
 // (ozaki.cu), used whenever the job holds b's slices (ozaki_build, once):
 // t1_ozaki computes tmp[m + nbf*q + nbf*nbf5*l] = (B_l C5)[m, q] in FP64; where
-// ozaki_products(job) (b's rows are of like size), T2 and Y run from digits too:
+// ozaki_products (b's rows are of like size, and not a few orbitals in a small basis),
+// T2 and Y run from digits too:
 // transforms_ozaki leaves tmp as digit slices in job->tmp and b_pq in job->bpq;
 // y_ozaki then builds W's slices and leaves FP64 partials of Y in job->part (the
 // coefficients given to both must be the same).
 bool ozaki_shape_ok(int nbf);
-bool ozaki_products(const donof_job* job);
+bool ozaki_products(const donof_job* job, int nbf5);
 size_t ozaki_bytes(int nbf, int naux);
 int ozaki_build(donof_job* job);
 void ozaki_free(donof_job* job);

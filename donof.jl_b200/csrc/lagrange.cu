@@ -216,7 +216,7 @@ int grid_for(long long total, int threads, int sm) {
 int transforms_f64(donof_job* job, cudaStream_t st, const double* C, int nbf5) {
     donof_ctx* ctx = job->ctx;
     const int nbf = job->nbf, naux = job->naux;
-    if (ozaki_products(job)) return transforms_ozaki(job, st, C, nullptr, nullptr, nullptr, nbf5);
+    if (ozaki_products(job, nbf5)) return transforms_ozaki(job, st, C, nullptr, nullptr, nullptr, nbf5);
     DONOF_CHECK(job->tmp.ensure(ctx, sizeof(double) * (size_t)nbf * nbf5 * naux));
     DONOF_CHECK(job->bpq.ensure(ctx, sizeof(double) * (size_t)nbf5 * nbf5 * naux));
     double* tmp = job->tmp.as<double>();
@@ -259,7 +259,7 @@ int y_partials(donof_job* job, cudaStream_t st, const double* C, const double* n
     const int nbf = job->nbf, naux = job->naux;
     unsigned* words = nullptr;
     DONOF_CHECK(tail_state(job, nbf5, &words));
-    if (ozaki_products(job)) {
+    if (ozaki_products(job, nbf5)) {
         DONOF_CHECK(transforms_ozaki(job, st, C, n, cj12, ck12, nbf5));
         return y_ozaki(job, st, n, cj12, ck12, nbf5, nalpha, nbeta, ypart, nparts, words);
     }

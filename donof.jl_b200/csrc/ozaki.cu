@@ -1221,7 +1221,15 @@ int t1(donof_job* job, cudaStream_t st, int nbf5, double* out) {
 
 }  // namespace
 
-bool ozaki_products(const donof_job* job) { return job->oz_b && !job->oz_t1_only; }
+// T2 and Y from digits, or as FP64 GEMMs of T1's tmp: those where b's rows differ too much
+// in size, and for a few orbitals in a small basis, where the digit route's launches and
+// the padding of nbf5 to 64 columns cost more than the products (Lagrangian and JKH_MO in
+// us at naux = 4 nbf: nbf = 128, nbf5 = 8 87 and 96 from digits, 69 and 91 as GEMMs; 200
+// and 24 152 and 137 against 137 and 127; but 200 and 32 154 and 139 against 152 and 131,
+// 200 and 48 174 and 145 against 191 and 146, 256 and 16 173 and 182 against 193 and 184).
+bool ozaki_products(const donof_job* job, int nbf5) {
+    return job->oz_b && !job->oz_t1_only && (nbf5 > 24 || job->nbf >= 224);
+}
 
 bool ozaki_shape_ok(int nbf) { return nbf >= 1 && nbf <= 16384; }
 

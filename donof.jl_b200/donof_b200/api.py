@@ -150,7 +150,8 @@ class BTensor:
         """Run the FP64 form's contractions on the tensor cores from int8 digit
         slices (b's made now, 7/8 of its FP64 size), or back on the FP64 GEMM
         (enable=False frees the slices).  Where b's row norms differ by more
-        than 64 times, the first contraction alone runs from digits."""
+        than 64 times, and for nbf5 <= 24 at nbf < 224 (faster so), the first
+        contraction alone runs from digits."""
         self.ctx.check(self.ctx.lib.donof_job_set_fp64_tc(self.handle, 1 if enable else 0))
 
     @property

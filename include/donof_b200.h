@@ -182,7 +182,8 @@ int donof_transform_dev(donof_job* job, int precision, const double* C, int nbf5
  * inside the form's 1e-10 parity.  tmp_l keeps that for every row of b_l by
  * itself.  b_pq and the sum hold their operands relative to the largest row
  * norm of b_l; where the row norms (each the largest over l) differ by more
- * than 64 times, they run as FP64 GEMMs of tmp_l instead.  enable = 0 frees the slices (the DMMA
+ * than 64 times, they run as FP64 GEMMs of tmp_l instead, as they do for
+ * nbf5 <= 24 at nbf < 224, where those are faster.  enable = 0 frees the slices (the DMMA
  * GEMM runs again).  Needs nbf <= 16384.  donof_job_fp64_tc tells
  * whether the slices are present.                                            */
 int donof_job_set_fp64_tc(donof_job* job, int enable);

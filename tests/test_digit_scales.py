@@ -75,7 +75,7 @@ def system(kind, orbitals, seed=3):
         b = b.reshape(nbf, nbf, naux, order="F")
         b = np.asfortranarray((b + b.transpose(1, 0, 2)) / 2)
         S = integrals.one_electron(orb)[0]
-    p = Param(nbf=nbf, nbfaux=naux, nalpha=5, nbeta=5, ncwo=3)
+    p = Param(nbf=nbf, nbfaux=naux, nalpha=7, nbeta=7, ncwo=3)
     if orbitals == "own":                 # the basis functions themselves, orthogonalised
         s, U = np.linalg.eigh(S)
         C = (U / np.sqrt(s)) @ U.T

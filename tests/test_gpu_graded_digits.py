@@ -36,7 +36,7 @@ def test_every_element_keeps_its_own_bound(cuda_ctx, kind, orbitals):
     assert np.all(np.abs(elag - e0)[:, :p.nbf5] <= eb)
 
 
-@pytest.mark.parametrize("nbf,naux,nbeta,ncwo,nopen", [(48, 20, 4, 3, 0), (129, 22, 16, 3, 1), (202, 37, 33, 5, 0),
+@pytest.mark.parametrize("nbf,naux,nbeta,ncwo,nopen", [(48, 20, 7, 3, 0), (129, 22, 16, 3, 1), (202, 37, 33, 5, 0),
                                                        (256, 30, 16, 3, 0), (300, 9, 20, 2, 0)])
 def test_t2_and_y_are_as_near_as_fp64_products_of_the_same_tmp(cuda_ctx, nbf, naux, nbeta, ncwo, nopen):
     """b_pq and elag against FP64 products of the tmp that T1 gives.  tmp, C5 and W are
