@@ -20,16 +20,25 @@ constexpr int JD = 512;          // largest nbf5 staged (32 KB)
 
 // (p, q) per thread: four with staged diagonals, or one with direct loads where there
 // are few blocks along (p, q) (four a thread would need more chunks of l, whose
-// partials a second kernel sums in order: JKH_MO at nbf5 = 60 62 us, 64 with staging).
-inline int per_thread(int nbf5) { return (long long)nbf5 * nbf5 >= 8192 ? 4 : 1; }
+// partials a second kernel sums in order: JKH_MO at nbf5 = 60 62 us, 64 with staging)
+// and where the diagonals are long (the kernel alone, four against one: FP32 at nbf5 =
+// 300, naux = 400 172 and 203 us, at 360 245 and 207, at 400 330 and 211; FP64 at 400
+// 240 and 212, at 450, naux = 200 146 and 215, at 512 226 and 214; beyond JD four with
+// direct loads took 304 and 137 us at 600, 200 and 100, in the two types, one 304 and 125).
+template <class T>
+int per_thread(int nbf5) {
+    return nbf5 <= (sizeof(T) == 4 ? 320 : JD) && (long long)nbf5 * nbf5 >= 8192 ? 4 : 1;
+}
 // blocks along (p, q); chunk of l for two or three blocks per SM
-inline int blocks(int nbf5) {
-    const long long span = (long long)per_thread(nbf5) * JT;
+template <class T>
+int blocks(int nbf5) {
+    const long long span = (long long)per_thread<T>(nbf5) * JT;
     return (int)(((long long)nbf5 * nbf5 + span - 1) / span);
 }
-inline int chunk(int nbf5, int naux, int sms) {
-    const int want = (per_thread(nbf5) == 4 ? 3 : 2) * sms;
-    int n = (want + blocks(nbf5) - 1) / blocks(nbf5);
+template <class T>
+int chunk(int nbf5, int naux, int sms) {
+    const int want = (per_thread<T>(nbf5) == 4 ? 3 : 2) * sms;
+    int n = (want + blocks<T>(nbf5) - 1) / blocks<T>(nbf5);
     if (n > naux) n = naux;
     if (n < 1) n = 1;
     return (naux + n - 1) / n;
@@ -62,7 +71,7 @@ __device__ __forceinline__ void stage_diagonals(const T* __restrict__ B, int nbf
 template <class T, int JE>
 __global__ void __launch_bounds__(JT) partial_kernel(const T* __restrict__ bpq, int nbf5, int naux, int lchunk,
                                                      double* __restrict__ part) {
-    __shared__ double sd[JL][JD];
+    __shared__ double sd[JE == 1 ? 1 : JL][JE == 1 ? 1 : JD];  // (32 KB would cost direct loads a block per SM)
     const long long n55 = (long long)nbf5 * nbf5, base = blockIdx.x * (long long)(JE * JT) + threadIdx.x;
     const int c = blockIdx.y;
     const int l0 = c * lchunk, l1 = min(naux, l0 + lchunk);
@@ -75,7 +84,7 @@ __global__ void __launch_bounds__(JT) partial_kernel(const T* __restrict__ bpq, 
         q[j] = i < n55 ? (int)(i / nbf5) : 0;
         sj[j] = sk[j] = 0.0;
     }
-    if (JE == 1 || nbf5 > JD) {
+    if (JE == 1) {
         for (int l = l0; l < l1; ++l) {
             const T* B = bpq + n55 * l;
 #pragma unroll
@@ -127,8 +136,8 @@ __global__ void __launch_bounds__(JT) partial_kernel(const T* __restrict__ bpq, 
 // The launch: grid (blocks, chunks).
 template <class T>
 void launch_partial(cudaStream_t st, const T* bpq, int nbf5, int naux, int lchunk, double* part) {
-    const dim3 grid(blocks(nbf5), (naux + lchunk - 1) / lchunk);
-    if (per_thread(nbf5) == 4) partial_kernel<T, 4><<<grid, JT, 0, st>>>(bpq, nbf5, naux, lchunk, part);
+    const dim3 grid(blocks<T>(nbf5), (naux + lchunk - 1) / lchunk);
+    if (per_thread<T>(nbf5) == 4) partial_kernel<T, 4><<<grid, JT, 0, st>>>(bpq, nbf5, naux, lchunk, part);
     else partial_kernel<T, 1><<<grid, JT, 0, st>>>(bpq, nbf5, naux, lchunk, part);
     count_launch();
 }

@@ -319,7 +319,7 @@ int jkh_mo_f64(donof_job* job, cudaStream_t st, const double* C, const double* H
     const int nbf = job->nbf, naux = job->naux;
     DONOF_CHECK(transforms_f64(job, st, C, nbf5));
     const long long n55 = (long long)nbf5 * nbf5;
-    const int lchunk = jk::chunk(nbf5, naux, ctx->sm_count);
+    const int lchunk = jk::chunk<double>(nbf5, naux, ctx->sm_count);
     const int chunks = (naux + lchunk - 1) / lchunk;
     DONOF_CHECK(job->part.ensure(ctx, sizeof(double) * (size_t)chunks * 2 * n55));
     double* part = job->part.as<double>();

@@ -685,7 +685,7 @@ int jkh_mo_mixed_general(donof_job* job, cudaStream_t st, const double* C, const
     DONOF_CHECK(gen_prepare(job, st, C, nullptr, nullptr, nullptr, nbf5, false, &S));
     DONOF_CHECK(gen_transforms(job, st, nbf5, S));
     const long long n55 = (long long)nbf5 * nbf5;
-    const int lchunk = jk::chunk(nbf5, naux, ctx->sm_count);
+    const int lchunk = jk::chunk<float>(nbf5, naux, ctx->sm_count);
     const int chunks = (naux + lchunk - 1) / lchunk;
     DONOF_CHECK(job->part.ensure(ctx, sizeof(double) * (size_t)chunks * 2 * n55));
     double* part = job->part.as<double>();
