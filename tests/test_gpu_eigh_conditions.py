@@ -55,8 +55,8 @@ def test_a_coulomb_metric(cuda_ctx):
     assert np.max(np.abs(build(cuda_ctx, G, I) - ref)) <= 2 * n * 2.0 ** -54 * w[-1] / w[0] * np.max(np.abs(ref))
 
 
-@pytest.mark.parametrize("n", [96, 320, 512])
-@pytest.mark.parametrize("kind", ["half rank", "repeated functions", "near zero"])
+@pytest.mark.parametrize("kind,n", [(k, n) for k in ("half rank", "repeated functions", "near zero")
+                                    for n in (96, 320, 512)] + [("eighteen decades", 1024)])
 def test_less_than_full_rank_ends(cuda_ctx, kind, n):
     """The sweeps end within their limit (rounding may leave an eigenvalue of exactly
     zero, whose b is refused as not finite).  In the space of the large eigenvalues b is
@@ -77,6 +77,8 @@ def test_less_than_full_rank_ends(cuda_ctx, kind, n):
         Q = np.linalg.qr(rng.standard_normal((n, n)))[0]
         w = np.linspace(0.5, 4.0, n)
         w[:n // 8] = np.linspace(-1e-13, 1e-13, n // 8)
+        if kind == "eighteen decades":
+            w = np.logspace(-18, 0, n)
         G = symmetric((Q * w) @ Q.T)
     I = rng.standard_normal((4, 4, n))
     try:
