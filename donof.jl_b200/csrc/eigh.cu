@@ -11,7 +11,8 @@
 // has two phases between bounded grid barriers (dtile.cuh):
 //   A  a CTA per block pair rotates the pair's 64 x 64 diagonal block in shared
 //      memory, accumulating the rotations in a 64 x 64 Q: in a sweep's first round
-//      all 63 x 32 index pairs (circle ordering), in the others the 32 x 32 pairs
+//      all 63 x 32 index pairs (circle ordering; those of a smaller matrix alone: Iaux
+//      at naux = 8 495 us with all of them, 224 so), in the others the 32 x 32 pairs
 //      across the two blocks (32 steps of 32 disjoint pairs).  A sweep visits
 //      every index pair outside the blocks once, and those inside once.
 //   B  the other 64 x 64 blocks of A become Q1^T A_blk Q2 and V's column pairs V Q,
@@ -65,12 +66,15 @@ struct EigArgs {
     double* Q;      // P matrices of 64 x 64 (column-major), the round's rotations
     int* rotated;   // P flags of the round
     EigState* st;
-    int N, P;       // padded size, block pairs
+    int n, N, P;    // size, padded size, block pairs
     dtile::WaitCtl wc;
 };
 
-// Index at position pos of round r of the circle ordering of n (position 0 fixed).
-__device__ __forceinline__ int circle(int pos, int r, int n) { return pos == 0 ? 0 : 1 + (pos - 1 + r) % (n - 1); }
+// Index at position pos of round r < n - 1 of the circle ordering of n (position 0 fixed).
+__device__ __forceinline__ int circle(int pos, int r, int n) {
+    const int x = pos + r;
+    return pos == 0 ? 0 : x < n ? x : x - (n - 1);
+}
 
 // Blocks I < J of pair p in round r.
 __device__ __forceinline__ void block_pair(int p, int r, int nb, int& I, int& J) {
@@ -215,12 +219,18 @@ __device__ void rotate_pair(const EigArgs& a, int p, int r, int sweep, double* s
     if (r == 0) {
         const int i = (tid - SW_THREADS) >> 1, j0 = EB / 2 * (tid & 1);  // row of Q, first rotation
         double* row = Q + i;
-        for (int k = 0; k < PB - 1; ++k) {
+        // (a matrix smaller than the block: the circle of its own indices, the others idle)
+        const int ring = a.P == 1 ? (a.n + 1) & ~1 : PB;
+        if (tid < EB && tid >= ring / 2) {
+            rcs[tid] = make_double2(1.0, 0.0);
+            rpq[tid] = 2 * tid | (2 * tid + 1) << 8;
+        }
+        for (int k = 0; k < ring - 1; ++k) {
             int act = 0;
-            if (tid < EB) act = form(circle(tid, k, PB), circle(PB - 1 - tid, k, PB));
+            if (tid < ring / 2) act = form(circle(tid, k, ring), circle(ring - 1 - tid, k, ring));
             if (!__syncthreads_or(act)) continue;
             if (tid < SW_THREADS) {
-                if (tid < EB) keep();
+                if (tid < ring / 2) keep();
                 apply();
             } else {
                 constexpr int U = 8;  // loads of U rotations before their stores
@@ -473,7 +483,7 @@ int eigh_jacobi(donof_ctx* ctx, cudaStream_t st, const double* G, int n, double*
     const int tiles = P * (P - 1) / 2 + P * (N / PB);
     int grid = ctx_ctas(ctx);  // at most one CTA per SM: co-resident (the kernel has grid barriers)
     if (grid > tiles) grid = tiles;
-    EigArgs a{A, V, Q, rotated, es, N, P, dtile::wait_ctl(ctx)};
+    EigArgs a{A, V, Q, rotated, es, n, N, P, dtile::wait_ctl(ctx)};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(EIG_THREADS);

@@ -37,6 +37,8 @@ __global__ void gmsqrt_factors_kernel(const double* __restrict__ V, const double
     }
 }
 
+constexpr size_t SMALL_COPY = size_t(256) << 10;  // bytes of I that cross on the call's own stream
+
 // Copies `bytes` of host memory to dst on the stream `st`, returning when they have
 // landed.  Page-locked memory goes in one DMA; other memory through the context's
 // page-locked buffer in chunks, each host thread filling two slots of its own in
@@ -159,16 +161,24 @@ int iaux_f64(donof_ctx* ctx, cudaStream_t st, const double* G_host, const double
     DONOF_CUDA(ctx, cudaMemcpyAsync(dG, G_host, sizeof(double) * na2, cudaMemcpyHostToDevice, st));
     // eigen-decomposition of Symmetric(G) (its upper triangle)
     // I crosses on a stream of its own meanwhile (8 waters: 151 MB, 14 ms by one host
-    // thread behind the solver, 4 ms by eight beside it; the solver takes 10 ms)
-    if (!ctx->aux_stream) DONOF_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
-    cudaEvent_t ready = nullptr;  // dI's allocation is ordered on st
-    DONOF_CUDA(ctx, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-    cudaError_t e = cudaEventRecord(ready, st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->aux_stream, ready, 0);
-    cudaEventDestroy(ready);
-    DONOF_CUDA(ctx, e);
+    // thread behind the solver, 4 ms by eight beside it; the solver takes 10 ms), but for
+    // an I that costs less than the stream's events and synchronisations (a call at nbf =
+    // 24, naux = 1: 141 us with them, 110 without)
+    const size_t ibytes = sizeof(double) * nn * naux;
+    const bool beside = ibytes > SMALL_COPY;
+    if (beside) {
+        if (!ctx->aux_stream) DONOF_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
+        cudaEvent_t ready = nullptr;  // dI's allocation is ordered on st
+        DONOF_CUDA(ctx, cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        cudaError_t e = cudaEventRecord(ready, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->aux_stream, ready, 0);
+        cudaEventDestroy(ready);
+        DONOF_CUDA(ctx, e);
+    } else {
+        DONOF_CUDA(ctx, cudaMemcpyAsync(dI, I_host, ibytes, cudaMemcpyHostToDevice, st));
+    }
     DONOF_CHECK(eigh_jacobi(ctx, st, dG, naux, dA, dV, dw, escr));
-    const int copied = upload(ctx, ctx->aux_stream, dI, I_host, sizeof(double) * nn * naux);
+    const int copied = beside ? upload(ctx, ctx->aux_stream, dI, I_host, ibytes) : DONOF_OK;
     const int solved = eigh_finish(ctx, st, escr);
     DONOF_CHECK(copied);
     DONOF_CHECK(solved);
