@@ -40,19 +40,19 @@ __global__ void gmsqrt_factors_kernel(const double* __restrict__ V, const double
 constexpr size_t SMALL_COPY = size_t(256) << 10;  // bytes of I that cross on the call's own stream
 
 // Copies `bytes` of host memory to dst on the stream `st`, returning when they have
-// landed.  Page-locked memory goes in one DMA; other memory through the context's
-// page-locked buffer in chunks, each host thread filling two slots of its own in
+// landed.  Memory that CUDA knows (page-locked, managed, on the device too) goes in one
+// copy; other memory through the context's page-locked buffer in chunks, each host thread filling two slots of its own in
 // turn: one thread copies about 10 GB/s, the DMA takes five times that.
 int upload(donof_ctx* ctx, cudaStream_t st, void* dst, const void* src, size_t bytes) {
     constexpr size_t CHUNK = size_t(4) << 20;
     constexpr int MAX_THREADS = 8;
     const size_t chunks = (bytes + CHUNK - 1) / CHUNK;
     cudaPointerAttributes at{};
-    bool locked = cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    const bool known = cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
     cudaGetLastError();
     int nt = (int)std::min<size_t>(std::min<size_t>(MAX_THREADS, std::thread::hardware_concurrency() / 2), chunks / 2);
     const size_t room = 2 * CHUNK * (size_t)std::max(nt, 0);
-    if (!locked && nt > 1) {
+    if (!known && nt > 1) {
         if (ctx->hstage_busy) {  // an earlier call that failed may still be copying through it
             DONOF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             ctx->hstage_busy = false;
@@ -69,7 +69,7 @@ int upload(donof_ctx* ctx, cudaStream_t st, void* dst, const void* src, size_t b
             }
         }
     }
-    if (locked || nt <= 1 || ctx->hstage_bytes < room) {
+    if (known || nt <= 1 || ctx->hstage_bytes < room) {
         DONOF_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         DONOF_CUDA(ctx, cudaStreamSynchronize(st));
         return DONOF_OK;
