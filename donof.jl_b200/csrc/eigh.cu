@@ -359,24 +359,26 @@ __device__ void update_tile(const EigArgs& a, int t, int r, double* sm) {
         __syncthreads();
         product(Q1, LD, 1, X, acc);  // T(i, j) = sum_k Q1(k, i) X(k, j)
         __syncthreads();
-        if (mine)
+        if (mine) {
 #pragma unroll
-        for (int n = 0; n < PN; ++n)
+            for (int n = 0; n < PN; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)  // T as [i][k]
-                X[(i0 + g + 8 * (e >> 1)) * LD + j0 + 8 * n + 2 * tq + (e & 1)] = acc[n][e];
+                for (int e = 0; e < 4; ++e)  // T as [i][k]
+                    X[(i0 + g + 8 * (e >> 1)) * LD + j0 + 8 * n + 2 * tq + (e & 1)] = acc[n][e];
+        }
         __syncthreads();
         product(X, LD, 1, Q2, acc);
-        if (mine)
+        if (mine) {
 #pragma unroll
-        for (int n = 0; n < PN; ++n)
+            for (int n = 0; n < PN; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int gi = global_index(i0 + g + 8 * (e >> 1), I1, J1);
-                const int gj = global_index(j0 + 8 * n + 2 * tq + (e & 1), I2, J2);
-                a.A[gi + N * gj] = acc[n][e];
-                a.A[gj + N * gi] = acc[n][e];
-            }
+                for (int e = 0; e < 4; ++e) {
+                    const int gi = global_index(i0 + g + 8 * (e >> 1), I1, J1);
+                    const int gj = global_index(j0 + 8 * n + 2 * tq + (e & 1), I2, J2);
+                    a.A[gi + N * gj] = acc[n][e];
+                    a.A[gj + N * gi] = acc[n][e];
+                }
+        }
     } else {
         const int v = t - nt, p = v % a.P, row0 = v / a.P * PB;
         if (!a.rotated[p]) return;
@@ -390,12 +392,13 @@ __device__ void update_tile(const EigArgs& a, int t, int r, double* sm) {
         }
         __syncthreads();
         product(X, 1, LD, Q1, acc);
-        if (mine)
+        if (mine) {
 #pragma unroll
-        for (int n = 0; n < PN; ++n)
+            for (int n = 0; n < PN; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                a.V[row0 + i0 + g + 8 * (e >> 1) + N * global_index(j0 + 8 * n + 2 * tq + (e & 1), I, J)] = acc[n][e];
+                for (int e = 0; e < 4; ++e)
+                    a.V[row0 + i0 + g + 8 * (e >> 1) + N * global_index(j0 + 8 * n + 2 * tq + (e & 1), I, J)] = acc[n][e];
+        }
     }
     __syncthreads();  // the buffers are free
 }

@@ -70,9 +70,6 @@ int gemm_f64_partials_splits(donof_ctx* ctx, cudaStream_t st, bool a_kmajor, boo
                              const double* A, long long lda, const double* B, long long ldb, DevBuf* part,
                              int* splits, int* kchunk);
 
-// Fused FP64 tail of the Lagrangian (tail.cu): Y = sum of nparts partials
-// (FP32 or FP64, part[g * pstride + m + nbf * b]), HC = H C5, H_mat = C^T HC,
-// elag = [n o H_mat + C^T Y | 0] and E_elec (when E != nullptr).
 // Launches a kernel that starts with gemm_detail::stream_order() so that its CTAs are
 // brought in while the kernel before it ends (programmatic dependent launch); in a
 // captured graph an ordinary launch.
@@ -106,6 +103,10 @@ __device__ __forceinline__ void zero_tail_state(unsigned* words) {
     if (words != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < TAIL_STATE_WORDS)
         words[threadIdx.x] = 0;
 }
+// Fused FP64 tail of the Lagrangian (tail.cu): Y = sum of nparts partials
+// (FP32 or FP64, part[g * pstride + m + nbf * b]), HC = H C5, H_mat = C^T HC,
+// elag = [n o H_mat + C^T Y | 0] and E_elec (when E != nullptr).
+// state_zeroed: a kernel of this call has zeroed the barrier state (above).
 int elag_tail_f64(donof_job* job, cudaStream_t st, const double* C, const double* H, const double* n, int nbf5,
                   const void* part, bool part_f32, int nparts, long long pstride, double* Hmat, double* elag,
                   double* E, bool state_zeroed = false);
