@@ -87,7 +87,9 @@ int donof_b_upload(donof_ctx* ctx, const double* b_host, int nbf, int naux, int 
  * integrals G (naux x naux, host, the upper triangle is read as
  * Symmetric(G)) and the three-centre integrals I (nbf x nbf x naux, host) it
  * builds b = I G^{-1/2} on the device (negative eigenvalues of G give zero
- * inverse square roots) and returns a job that owns it, as donof_b_upload. */
+ * inverse square roots) and returns a job that owns it, as donof_b_upload.
+ * An I of 16 MB and more in ordinary memory crosses through up to 64 MB of
+ * page-locked memory, which the context keeps for later calls.               */
 int donof_iaux(donof_ctx* ctx, const double* G, const double* I3c, int nbf, int naux, int precision,
                donof_job** job);
 int donof_b_attach(donof_ctx* ctx, const double* b_dev, int nbf, int naux, int precision,
